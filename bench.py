@@ -70,7 +70,7 @@ def log(*a):
 # ------------------------------------------------------------------ traffic
 
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "transport_fast_traffic.json")
-KERNEL_SOURCES = ("transport.cuh", "transport_fast.cu", "engine_types.h", "portable_math.h")
+KERNEL_SOURCES = ("transport.cuh", "walk.cuh", "transport_fast.cu", "engine_types.h", "portable_math.h")
 
 
 def kernel_source_sha() -> str:

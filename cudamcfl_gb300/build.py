@@ -37,7 +37,7 @@ CUDA_UNITS = {
     "noalloc.cu": EXACT,
 }
 HOST_UNITS = ["engine.cpp", "run.cpp", "mci.cpp", "safeprimes.cpp", "server.cpp", "tune.cpp"]
-HEADERS = ["engine_types.h", "portable_math.h", "mcfl_internal.h", "transport.cuh"]
+HEADERS = ["engine_types.h", "portable_math.h", "mcfl_internal.h", "transport.cuh", "walk.cuh"]
 
 
 def _cuda_home() -> str:

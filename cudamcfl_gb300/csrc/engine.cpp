@@ -254,6 +254,29 @@ extern "C" unsigned long long mcfl_launch_count(const mcfl_ctx *c) { return c ? 
 
 /* ------------------------------------------------------------------ media */
 
+/* Whether the walk kernel (walk.cuh) runs a medium with the label records
+ * `lab`: the grid holds only labels 1..n_bulks, and these scatter, are not
+ * isotropic, share one refractive index and drop between a little and half of
+ * a weight per pass, so that no pass inside the slab needs a decision.
+ * w_event: a larger weight is still above the roulette's threshold (429497,
+ * CUDAMCFL.h:33) after one drop of any label; 1.0001 covers the drop's
+ * roundings. */
+static bool walk_limits(const mcfl_medium *m, const float *lab, unsigned lab_min, unsigned lab_max,
+                        uint32_t *w_event) {
+  const int n = m->n_bulks;
+  bool ok = lab_min >= 1u && lab_max <= (unsigned)n && lab[0] == FLT_MAX &&
+            lab[MCFL_LAB_FLOATS * (size_t)(n + 1)] == FLT_MAX;
+  float drop = 0.0f;
+  for (int i = 1; i <= n; ++i) {
+    const float *t = lab + MCFL_LAB_FLOATS * (size_t)i;
+    drop = std::max(drop, t[1]);
+    ok = ok && t[0] > 0.0f && t[0] < FLT_MAX && t[1] >= 1e-30f && t[1] <= 0.5f && t[4] != 0.0f &&
+         t[7] == lab[MCFL_LAB_FLOATS + 7];
+  }
+  *w_event = ok ? (uint32_t)(429501.0 / (1.0 - 1.0001 * (double)drop)) + 8u : 0u;
+  return ok;
+}
+
 extern "C" int mcfl_medium_create(mcfl_ctx *c, const mcfl_medium_desc *d, mcfl_medium **out) {
   if (!c || !d || !out || !d->labels || !d->bulks) return fail(MCFL_E_ARG, "mcfl_medium_create: null argument");
   *out = nullptr;
@@ -262,8 +285,12 @@ extern "C" int mcfl_medium_create(mcfl_ctx *c, const mcfl_medium_desc *d, mcfl_m
   if (total >= 0xFFFFFFFFull) return fail(MCFL_E_RANGE, "medium: more than 2^32-1 voxels");
   if (d->n_bulks < 1 || d->n_bulks > MCFL_MAX_BULKS) return fail(MCFL_E_RANGE, "medium: n_bulks out of range");
   if (!(d->half_x > 0 && d->half_y > 0 && d->thickness > 0)) return fail(MCFL_E_ARG, "medium: non-positive extent");
-  for (unsigned long long i = 0; i < total; ++i)
-    if (d->labels[i] > (unsigned)d->n_bulks + 1u) return fail(MCFL_E_ARG, "medium: label beyond n_bulks+1");
+  unsigned lab_min = 255, lab_max = 0;
+  for (unsigned long long i = 0; i < total; ++i) {
+    lab_min = std::min<unsigned>(lab_min, d->labels[i]);
+    lab_max = std::max<unsigned>(lab_max, d->labels[i]);
+  }
+  if (lab_max > (unsigned)d->n_bulks + 1u) return fail(MCFL_E_ARG, "medium: label beyond n_bulks+1");
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   mcfl_medium *m = new mcfl_medium();
   m->serial = next_medium_serial();
@@ -304,6 +331,8 @@ extern "C" int mcfl_medium_create(mcfl_ctx *c, const mcfl_medium_desc *d, mcfl_m
     mcfl_label_record(tx, b.mua, b.g, b.n, &lex[MCFL_LAB_FLOATS * (size_t)i]);
     mcfl_label_record(tm, b.muaf, b.g, b.n, &lmx[MCFL_LAB_FLOATS * (size_t)i]);
   }
+  m->plain[0] = walk_limits(m, le.data(), lab_min, lab_max, &m->w_event[0]);
+  m->plain[1] = walk_limits(m, lm.data(), lab_min, lab_max, &m->w_event[1]);
   cudaError_t e = m->labels.reserve(total);
   if (e == cudaSuccess) e = cudaMemcpyAsync(m->labels.p, d->labels, total, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = m->prop_exc.reserve(pe.size() * 4);

@@ -180,6 +180,10 @@ typedef struct McflLaunch {
   /* lanes of a warp without a photon wait until at least this many are
    * free (or every lane is), then draw new photons together (0: 1) */
   uint32_t relaunch_min;
+  /* plain: every medium of the launch is plain (mcfl_medium::plain), so the
+   * walk kernel runs it; w_event: the weight up to which it takes the event
+   * code; sm_count: the GPU's SMs */
+  uint32_t plain, w_event, sm_count;
   float l2_hit_ratio;      /* host side: persisting-L2 window over [l2_base, +l2_bytes) when l2_bytes > 0 */
   const void *l2_base;
   unsigned long long l2_bytes;

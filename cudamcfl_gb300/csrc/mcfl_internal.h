@@ -129,6 +129,10 @@ struct mcfl_medium {
   int n_bulks = 0;
   bool has_fmap = false;
   std::vector<mcfl_bulk> bulks;
+  /* for the walk kernel's launches (McflLaunch::plain and w_event), by
+   * phase (excitation, emission): see walk_limits in engine.cpp */
+  bool plain[2] = {false, false};
+  uint32_t w_event[2] = {0, 0};
   size_t bytes = 0;
   /* layered medium (bulk method 1) */
   bool layered = false;

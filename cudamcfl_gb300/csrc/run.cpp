@@ -220,7 +220,15 @@ McflLaunch base_launch(mcfl_ctx *c) {
   L.step_cap = c->step_cap;
   L.variant = (uint32_t)c->variant_code();
   L.relaunch_min = c->relaunch;
+  L.sm_count = (uint32_t)c->sm_count;
   return L;
+}
+
+/* A mixed-media launch takes up medium m: it is plain when all its media are,
+ * its event weight the largest (L.plain starts as 1, L.w_event as 0). */
+void add_walk_limits(McflLaunch &L, const mcfl_medium *m) {
+  if (!m->plain[0]) L.plain = 0;
+  L.w_event = std::max(L.w_event, m->w_event[0]);
 }
 
 /* Every job of the launch uses medium m with one photon-hitting-density
@@ -240,6 +248,8 @@ void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool em
   u.lab = m->lab_of(emission, exact);
   u.lab16 = exact ? m->lab16.as<uint16_t>() : nullptr;
   u.n_labels = (uint32_t)m->n_bulks + 2u;
+  L.plain = m->plain[emission] ? 1u : 0u;
+  L.w_event = m->w_event[emission];
   u.fhd = fhd;
   u.hx = m->hx;
   u.hy = m->hy;
@@ -597,6 +607,11 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
   int block = 0, block_one = 0;
   const int grid = c->grid_for(uniform, &block, nullptr, timed, exact);
   float ms = 0.f;
+  McflLaunch limits; /* of a mixed-media launch */
+  limits.plain = 1;
+  limits.w_event = 0;
+  if (!uniform)
+    for (int i = 0; i < n; ++i) add_walk_limits(limits, media[i]);
   if (schedule == MCFL_SCHEDULE_BATCHED) {
     auto record = [&](cudaStream_t st, unsigned *k) -> cudaError_t {
       cudaError_t e;
@@ -612,7 +627,11 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
       L.ticket_counter = c->bcnt.as<unsigned long long>();
       L.ticket_end = tickets;
       if (uniform) set_uniform(c, L, m, false, nullptr, exact);
-      else L.variant = (uint32_t)c->mixed_code();
+      else {
+        L.variant = (uint32_t)c->mixed_code();
+        L.plain = limits.plain;
+        L.w_event = limits.w_event;
+      }
       L.exact_step = exact ? 1u : 0u;
       L.time_on = timed ? 1u : 0u;
       if ((e = record_event(c->ev[0], st))) return e;
@@ -628,7 +647,7 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
                 {N, xy, tickets, (unsigned long long)c->math, (unsigned long long)grid, (unsigned long long)block,
                  c->step_cap, (unsigned long long)c->variant_code(), (unsigned long long)c->l2_window,
                  (unsigned long long)uniform, (unsigned long long)exact, m->serial, tsize,
-                 (unsigned long long)c->mixed_code(), c->relaunch});
+                 (unsigned long long)c->mixed_code(), c->relaunch, limits.plain, limits.w_event});
     const int rcb = replay(c, &c->graph_batch, &c->graph_batch_key, &c->graph_batch_kernels, key, record);
     if (rcb != MCFL_OK) return rcb;
     MCFL_CUDA_TRY(cudaStreamSynchronize(s));

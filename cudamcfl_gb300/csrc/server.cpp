@@ -383,6 +383,13 @@ void mcfl_server::loop() {
     L.saved = parked[mode].as<McflSaved>();
     L.step_cap = ctx->step_cap;
     L.relaunch_min = ctx->relaunch;
+    L.sm_count = (uint32_t)ctx->sm_count;
+    L.plain = 1;
+    for (unsigned i = 0; i < slots; ++i)
+      if (active[i] && active[i]->mode == mode) {
+        if (!active[i]->medium->plain[0]) L.plain = 0;
+        L.w_event = std::max(L.w_event, active[i]->medium->w_event[0]);
+      }
     cudaMemsetAsync(stop_word.p, 0, 4, s);
     cudaEventRecord(ev_reset, s);
     {

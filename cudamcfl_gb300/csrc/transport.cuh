@@ -89,6 +89,7 @@ struct __align__(16) real4 {
 #define MCFL_R2U_RU(x) __double2uint_ru(x)
 #define MCFL_R2U_RN(x) __double2uint_rn(x)
 #define MCFL_KERNEL_NAME mcfl_transport_f64
+#define MCFL_WALK_NAME mcfl_transport_f64_walk
 #define MCFL_LAUNCHER mcfl_launch_transport_f64
 #define MCFL_ATTR_FN mcfl_attr_transport_f64
 #else
@@ -111,6 +112,7 @@ typedef float4 real4;
 #define MCFL_COSF(x) mcfl_pcosf(x)
 #define MCFL_RSQRTF(x) (1.0f / sqrtf(x))
 #define MCFL_KERNEL_NAME mcfl_transport_exact
+#define MCFL_WALK_NAME mcfl_transport_exact_walk
 #define MCFL_LAUNCHER mcfl_launch_transport_exact
 #define MCFL_ATTR_FN mcfl_attr_transport_exact
 #else
@@ -119,6 +121,7 @@ typedef float4 real4;
 #define MCFL_COSF(x) __cosf(x)
 #define MCFL_RSQRTF(x) rsqrtf(x)
 #define MCFL_KERNEL_NAME mcfl_transport_fast
+#define MCFL_WALK_NAME mcfl_transport_fast_walk
 #define MCFL_LAUNCHER mcfl_launch_transport_fast
 #define MCFL_ATTR_FN mcfl_attr_transport_fast
 #endif
@@ -720,6 +723,10 @@ __device__ __noinline__ void tally_time(const McflJob *J, real px, real py, uint
     }
   }
 }
+
+#if !MCFL_F64
+#include "walk.cuh"
+#endif
 
 } // namespace
 
@@ -1467,26 +1474,21 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
   flush_stats();
 }
 
-/* dynamic shared memory of a launch (threads: the variant's block size) */
-static size_t smem_bytes(int threads, bool uniform) {
-  (void)threads;
-  return lab_bytes(uniform) + 16;
-}
-
 /* Kernel variants.  Single medium (occupancy variants: threads per block x
  * the blocks per SM the register budget is cut for): 0 = 256 x 4,
  * 1 = 256 x 5, 2 = 128 x 9, chosen by the autotuner, and 7, 8, 9 the same
  * with the photon-hitting-density sums held in a register, 11, 12, 13 the
  * same with the pass in its per-test branching form, 14, 15, 16 the same
- * with the hitting-density adds aggregated per warp, 17, 18, 19 the same
- * as 0, 1, 2 with no hitting-density code (the launcher runs them for
- * launches that tally none: emission, excitation without fluence); 3 = 256 x 3 carrying
+ * with the hitting-density adds aggregated per warp; 3 = 256 x 3 carrying
  * the time of flight; layered medium 4 = 256 x 4, 5 = 256 x 3 with the time
  * of flight; voxel-boundary stepping 6 = 256 x 4, 10 = 256 x 3 with the time
  * of flight.  Mixed media: -1 = 256 x 3, -3 = 256 x 4, -4 = 128 x 7,
  * -5, -6, -7 the same with the per-test branching pass, -2 = 256 x 2 with
  * the time of flight; voxel-boundary stepping -8 = 256 x 3, -9 = 256 x 2 with
- * the time of flight. */
+ * the time of flight.  Launches over plain media run -4..3 as the walk kernel
+ * (walk.cuh).  0..2, and the walk kernel's, have instantiations with no
+ * hitting-density code for launches that tally none (emission, excitation
+ * without fluence). */
 typedef void (*TransportKernel)(McflLaunch);
 
 /* Mixed-media occupancy variants: 0 = 256 x 3, 1 = 256 x 4, 2 = 128 x 7;
@@ -1496,39 +1498,77 @@ static int mixed_variant_code(uint32_t v) {
   return v < 6 ? code[v] : -1;
 }
 
-static TransportKernel kernel_of(int variant, int *threads) {
+#if MCFL_F64
+/* the double-precision build runs the transport kernel's own pass throughout */
+static bool is_walk(int, bool) { return false; }
+static TransportKernel walk_of(int, bool) { return nullptr; }
+#else
+static bool is_walk(int variant, bool plain) { return plain && variant >= -4 && variant <= 3; }
+
+static TransportKernel walk_of(int variant, bool no_phd) {
   switch (variant) {
-  case -2: *threads = 256; return MCFL_KERNEL_NAME<false, true, 0, 256, 2>;
-  case -1: *threads = 256; return MCFL_KERNEL_NAME<false, false, 0, 256, 3>;
-  case -3: *threads = 256; return MCFL_KERNEL_NAME<false, false, 0, 256, 4>;
-  case -4: *threads = 128; return MCFL_KERNEL_NAME<false, false, 0, 128, 7>;
-  case -5: *threads = 256; return MCFL_KERNEL_NAME<false, false, 0, 256, 3, false, true>;
-  case -6: *threads = 256; return MCFL_KERNEL_NAME<false, false, 0, 256, 4, false, true>;
+  case -2: return MCFL_WALK_NAME<false, true, false, 256, 2>;
+  case -1: return MCFL_WALK_NAME<false, false, false, 256, 3>;
+  case -3: return MCFL_WALK_NAME<false, false, false, 256, 4>;
+  case -4: return MCFL_WALK_NAME<false, false, false, 128, 7>;
+  case 0: return no_phd ? MCFL_WALK_NAME<true, false, true, 256, 4> : MCFL_WALK_NAME<true, false, false, 256, 4>;
+  case 1: return no_phd ? MCFL_WALK_NAME<true, false, true, 256, 5> : MCFL_WALK_NAME<true, false, false, 256, 5>;
+  case 2: return no_phd ? MCFL_WALK_NAME<true, false, true, 128, 9> : MCFL_WALK_NAME<true, false, false, 128, 9>;
+  case 3: return MCFL_WALK_NAME<true, true, false, 256, 3>;
+  default: return nullptr;
+  }
+}
+#endif
+
+static TransportKernel kernel_of(int variant, int *threads, bool plain = false, bool no_phd = false) {
+  *threads = variant == -4 || variant == 2 ? 128 : 256;
+  if (is_walk(variant, plain)) return walk_of(variant, no_phd);
+  switch (variant) {
+  case -2: return MCFL_KERNEL_NAME<false, true, 0, 256, 2>;
+  case -1: return MCFL_KERNEL_NAME<false, false, 0, 256, 3>;
+  case -3: return MCFL_KERNEL_NAME<false, false, 0, 256, 4>;
+  case -4: return MCFL_KERNEL_NAME<false, false, 0, 128, 7>;
+  case 0:
+    return no_phd ? MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, false, false, true>
+                  : MCFL_KERNEL_NAME<true, false, 0, 256, 4>;
+  case 1:
+    return no_phd ? MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, false, false, true>
+                  : MCFL_KERNEL_NAME<true, false, 0, 256, 5>;
+  case 2:
+    return no_phd ? MCFL_KERNEL_NAME<true, false, 0, 128, 9, false, false, false, true>
+                  : MCFL_KERNEL_NAME<true, false, 0, 128, 9>;
+  case 3: return MCFL_KERNEL_NAME<true, true, 0, 256, 3>;
+  case -5: return MCFL_KERNEL_NAME<false, false, 0, 256, 3, false, true>;
+  case -6: return MCFL_KERNEL_NAME<false, false, 0, 256, 4, false, true>;
   case -7: *threads = 128; return MCFL_KERNEL_NAME<false, false, 0, 128, 7, false, true>;
-  case -8: *threads = 256; return MCFL_KERNEL_NAME<false, false, 2, 256, 3>;
-  case -9: *threads = 256; return MCFL_KERNEL_NAME<false, true, 2, 256, 2>;
-  case 0: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 4>;
-  case 1: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 5>;
-  case 2: *threads = 128; return MCFL_KERNEL_NAME<true, false, 0, 128, 9>;
-  case 3: *threads = 256; return MCFL_KERNEL_NAME<true, true, 0, 256, 3>;
-  case 4: *threads = 256; return MCFL_KERNEL_NAME<true, false, 1, 256, 4>;
-  case 5: *threads = 256; return MCFL_KERNEL_NAME<true, true, 1, 256, 3>;
-  case 6: *threads = 256; return MCFL_KERNEL_NAME<true, false, 2, 256, 4>;
-  case 7: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 4, true>;
-  case 8: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 5, true>;
+  case -8: return MCFL_KERNEL_NAME<false, false, 2, 256, 3>;
+  case -9: return MCFL_KERNEL_NAME<false, true, 2, 256, 2>;
+  case 4: return MCFL_KERNEL_NAME<true, false, 1, 256, 4>;
+  case 5: return MCFL_KERNEL_NAME<true, true, 1, 256, 3>;
+  case 6: return MCFL_KERNEL_NAME<true, false, 2, 256, 4>;
+  case 7: return MCFL_KERNEL_NAME<true, false, 0, 256, 4, true>;
+  case 8: return MCFL_KERNEL_NAME<true, false, 0, 256, 5, true>;
   case 9: *threads = 128; return MCFL_KERNEL_NAME<true, false, 0, 128, 9, true>;
-  case 10: *threads = 256; return MCFL_KERNEL_NAME<true, true, 2, 256, 3>;
-  case 11: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, true>;
-  case 12: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, true>;
+  case 10: return MCFL_KERNEL_NAME<true, true, 2, 256, 3>;
+  case 11: return MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, true>;
+  case 12: return MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, true>;
   case 13: *threads = 128; return MCFL_KERNEL_NAME<true, false, 0, 128, 9, false, true>;
-  case 14: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, false, true>;
-  case 15: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, false, true>;
+  case 14: return MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, false, true>;
+  case 15: return MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, false, true>;
   case 16: *threads = 128; return MCFL_KERNEL_NAME<true, false, 0, 128, 9, false, false, true>;
-  case 17: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 4, false, false, false, true>;
-  case 18: *threads = 256; return MCFL_KERNEL_NAME<true, false, 0, 256, 5, false, false, false, true>;
-  case 19: *threads = 128; return MCFL_KERNEL_NAME<true, false, 0, 128, 9, false, false, false, true>;
   default: *threads = 0; return nullptr;
   }
+}
+
+/* dynamic shared memory of a transport-kernel launch */
+static size_t smem_bytes(bool uniform) { return lab_bytes(uniform) + 16; }
+
+/* The L1/shared split [%]: just the shared memory that bps blocks need (1 KB
+ * per block is reserved by the system), the rest as L1 (the label gather of
+ * every pass hits it). */
+static int carveout(int max_sm, int bps, size_t smem) {
+  const size_t need = (size_t)bps * (smem + 1024);
+  return (int)std::min<size_t>(100, (need * 100 + (size_t)max_sm - 1) / (size_t)max_sm + 1);
 }
 
 /* Launches the kernel the launch asks for (single medium: L->variant, or
@@ -1549,29 +1589,46 @@ extern "C" cudaError_t MCFL_LAUNCHER(const McflLaunch *L, int grid, int block, c
                 : L->time_on        ? -2
                                     : mixed_variant_code(L->variant);
   int t = 0;
-  /* variants 0..2 without a hitting-density tally: their instantiations
-   * that compile none (17..19) */
-  const int vk = (v >= 0 && v <= 2 && !L->med.fhd) ? v + 17 : v;
-  const TransportKernel fn = kernel_of(vk, &t);
+  /* variants 0..2 without a hitting-density tally run their instantiations
+   * that compile none */
+  const bool no_phd = v >= 0 && v <= 2 && !L->med.fhd;
+  const TransportKernel fn = kernel_of(v, &t, L->plain != 0, no_phd);
   if (!fn || block > t) return cudaErrorInvalidValue;
+  const bool walk = is_walk(v, L->plain != 0);
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem_bytes(t, L->uniform_medium != 0);
+  cfg.dynamicSmemBytes = smem_bytes(L->uniform_medium != 0);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  memset(attr, 0, sizeof(attr));
   if (L->l2_bytes) {
-    memset(attr, 0, sizeof(attr));
-    attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-    attr[0].val.accessPolicyWindow.base_ptr = const_cast<void *>(L->l2_base);
-    attr[0].val.accessPolicyWindow.num_bytes = (size_t)L->l2_bytes;
-    attr[0].val.accessPolicyWindow.hitRatio = L->l2_hit_ratio;
-    attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
-    attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+    a.id = cudaLaunchAttributeAccessPolicyWindow;
+    a.val.accessPolicyWindow.base_ptr = const_cast<void *>(L->l2_base);
+    a.val.accessPolicyWindow.num_bytes = (size_t)L->l2_bytes;
+    a.val.accessPolicyWindow.hitRatio = L->l2_hit_ratio;
+    a.val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
+    a.val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
   }
+#if !MCFL_F64
+  if (walk) {
+    const bool timed = v == 3 || v == -2;
+    cfg.dynamicSmemBytes = walk_dynamic(v >= 0, timed, no_phd, block, L->med.n_labels);
+    int dev = 0, max_sm = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&max_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
+    if (max_sm > 0 && L->sm_count) {
+      cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+      a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+      a.val.sharedMemCarveout = (unsigned)carveout(max_sm, (grid + (int)L->sm_count - 1) / (int)L->sm_count,
+                                                   walk_static(t) + cfg.dynamicSmemBytes);
+    }
+  }
+#endif
+  cfg.attrs = cfg.numAttrs ? attr : nullptr;
   return cudaLaunchKernelEx(&cfg, fn, *L);
 }
 
@@ -1587,10 +1644,8 @@ extern "C" cudaError_t MCFL_ATTR_FN(int variant, int *block, int *blocks_per_sm,
   if (e != cudaSuccess) return e;
   if (regs) *regs = a.numRegs;
   if (*block <= 0 || *block > t) *block = t;
-  const size_t smem = smem_bytes(t, variant >= 0);
-  /* The L1/shared split: just the shared memory the blocks that the
-   * registers allow need, the rest as L1 (the label gather of every pass
-   * hits it).  Occupancy first with the whole shared memory available. */
+  const size_t smem = smem_bytes(variant >= 0);
+  /* occupancy with the whole shared memory available */
   e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
@@ -1601,14 +1656,13 @@ extern "C" cudaError_t MCFL_ATTR_FN(int variant, int *block, int *blocks_per_sm,
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&max_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
   if (bps > 0 && max_sm > 0) {
-    const size_t need = (size_t)bps * (smem + a.sharedSizeBytes + 1024); /* 1 KB per block reserved by the system */
-    const int pct = (int)std::min<size_t>(100, (need * 100 + (size_t)max_sm - 1) / (size_t)max_sm + 1);
-    e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             carveout(max_sm, bps, smem + a.sharedSizeBytes));
     if (e != cudaSuccess) return e;
     if (variant >= 0 && variant <= 2) { /* the same split for its instantiation without the tally */
-      int t2 = 0;
-      e = cudaFuncSetAttribute((const void *)kernel_of(variant + 17, &t2), cudaFuncAttributePreferredSharedMemoryCarveout,
-                               pct);
+      e = cudaFuncSetAttribute((const void *)kernel_of(variant, &t, false, true),
+                               cudaFuncAttributePreferredSharedMemoryCarveout,
+                               carveout(max_sm, bps, smem + a.sharedSizeBytes));
       if (e != cudaSuccess) return e;
     }
   }
