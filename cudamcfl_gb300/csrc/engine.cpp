@@ -273,8 +273,25 @@ static bool walk_limits(const mcfl_medium *m, const float *lab, unsigned lab_min
     ok = ok && t[0] > 0.0f && t[0] < FLT_MAX && t[1] >= 1e-30f && t[1] <= 0.5f && t[4] != 0.0f &&
          t[7] == lab[MCFL_LAB_FLOATS + 7];
   }
+  /* a coordinate inside the extent rounds to an index of the grid or onto its
+   * far face: one voxel of padding in the tiles holds it */
+  ok = ok && (m->hx + m->hx) * m->gx < (float)m->nx + 1.0f && (m->hy + m->hy) * m->gy < (float)m->ny + 1.0f &&
+       m->esp * m->gz < (float)m->nz + 1.0f && m->gx > 0.0f && m->gy > 0.0f && m->gz > 0.0f &&
+       tile_bytes_of(m->nx, m->ny, m->nz) < 0xFFFFFFFFull;
   *w_event = ok ? (uint32_t)(429501.0 / (1.0 - 1.0001 * (double)drop)) + 8u : 0u;
   return ok;
+}
+
+/* The smallest and the largest label of a grid (O3: the loop is vectorized). */
+__attribute__((optimize("O3"))) static void label_range(const unsigned char *labels, unsigned long long n,
+                                                        unsigned char *lo, unsigned char *hi) {
+  unsigned char a = 255, b = 0;
+  for (unsigned long long i = 0; i < n; ++i) {
+    a = labels[i] < a ? labels[i] : a;
+    b = labels[i] > b ? labels[i] : b;
+  }
+  *lo = a;
+  *hi = b;
 }
 
 extern "C" int mcfl_medium_create(mcfl_ctx *c, const mcfl_medium_desc *d, mcfl_medium **out) {
@@ -285,11 +302,8 @@ extern "C" int mcfl_medium_create(mcfl_ctx *c, const mcfl_medium_desc *d, mcfl_m
   if (total >= 0xFFFFFFFFull) return fail(MCFL_E_RANGE, "medium: more than 2^32-1 voxels");
   if (d->n_bulks < 1 || d->n_bulks > MCFL_MAX_BULKS) return fail(MCFL_E_RANGE, "medium: n_bulks out of range");
   if (!(d->half_x > 0 && d->half_y > 0 && d->thickness > 0)) return fail(MCFL_E_ARG, "medium: non-positive extent");
-  unsigned lab_min = 255, lab_max = 0;
-  for (unsigned long long i = 0; i < total; ++i) {
-    lab_min = std::min<unsigned>(lab_min, d->labels[i]);
-    lab_max = std::max<unsigned>(lab_max, d->labels[i]);
-  }
+  unsigned char lab_min = 255, lab_max = 0;
+  label_range(d->labels, total, &lab_min, &lab_max);
   if (lab_max > (unsigned)d->n_bulks + 1u) return fail(MCFL_E_ARG, "medium: label beyond n_bulks+1");
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   mcfl_medium *m = new mcfl_medium();

@@ -205,6 +205,33 @@ extern "C" cudaError_t mcfl_launch_normalize_128(const unsigned long long *raw, 
   return cudaGetLastError();
 }
 
+/* ------------------------------------------------ label tiles
+ * The walk kernel's label gather follows a photon whose steps are about half
+ * a voxel long in any direction.  With x fastest, a step in y or z lands in
+ * another cache line; in tiles of 4 x 4 voxels in y and z with x outside, a
+ * 32-byte sector holds 2 x 4 x 4 voxels and a line 8 x 4 x 4.  The padding
+ * voxel at each far face stands for coordinates that round up onto the face:
+ * it holds what the x-fastest index of that coordinate reads. */
+namespace {
+__global__ void tile_labels(const uint8_t *__restrict__ labels, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t total,
+                            uint8_t *__restrict__ tiles, uint32_t n) {
+  const uint32_t px = nx + 1u, by = ny / 4u + 1u;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const uint32_t t = (uint32_t)(i >> 4), w = (uint32_t)i & 15u;
+    const uint32_t x = t % px, y = (t / px) % by * 4u + (w >> 2), z = t / px / by * 4u + (w & 3u);
+    const uint32_t v = x + nx * (y + ny * z);
+    tiles[i] = labels[v < total ? v : total - 1u];
+  }
+}
+} // namespace
+
+extern "C" cudaError_t mcfl_launch_tiles(const uint8_t *labels, int nx, int ny, int nz, uint32_t total, uint8_t *tiles,
+                                         uint32_t tile_bytes, cudaStream_t s) {
+  tile_labels<<<grid_for(tile_bytes), 256, 0, s>>>(labels, (uint32_t)nx, (uint32_t)ny, (uint32_t)nz, total, tiles,
+                                                   tile_bytes);
+  return cudaGetLastError();
+}
+
 /* ------------------------------------------------ free-radius map
  * For voxel-boundary stepping: the free radius of a voxel is the largest
  * r <= MCFL_FREE_MAX such that every voxel of the grid within Chebyshev

@@ -143,6 +143,11 @@ typedef struct McflMedium {
    * free radius being the largest r <= MCFL_FREE_MAX such that every voxel
    * of the grid within Chebyshev distance r carries the same label */
   const uint16_t *lab16;
+  /* the walk kernel: the labels in tiles of 4 x 4 voxels in y and z, x outside
+   * (tiles: index ix*16 + iy*4 + iz + (iy/4)*tile_y + (iz/4)*tile_z, one
+   * voxel of padding at the far faces; tile_bytes of them) */
+  const uint8_t *tiles;
+  uint32_t tile_y, tile_z, tile_bytes, pad1;
 } McflMedium;
 
 #define MCFL_FREE_MAX 31

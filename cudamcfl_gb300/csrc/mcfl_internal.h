@@ -53,6 +53,13 @@ size_t emission_prep_blocks(uint32_t total);
 /* label | free radius << 8 per voxel (McflMedium::lab16); tmp: 2 * nx*ny*nz bytes */
 extern "C" cudaError_t mcfl_launch_free_map(const uint8_t *labels, int nx, int ny, int nz, uint8_t *tmp,
                                            uint16_t *lab16, cudaStream_t s);
+/* the labels in the walk kernel's tiles (McflMedium::tiles) */
+extern "C" cudaError_t mcfl_launch_tiles(const uint8_t *labels, int nx, int ny, int nz, uint32_t total, uint8_t *tiles,
+                                         uint32_t tile_bytes, cudaStream_t s);
+/* bytes of the tiles of a grid */
+inline unsigned long long tile_bytes_of(int nx, int ny, int nz) {
+  return 16ull * (unsigned long long)(nx + 1) * (unsigned long long)(ny / 4 + 1) * (unsigned long long)(nz / 4 + 1);
+}
 extern "C" cudaError_t mcfl_launch_normalize_u64(const unsigned long long *raw, double *out, size_t n, double scale,
                                                  cudaStream_t s);
 extern "C" cudaError_t mcfl_launch_normalize_phd(const unsigned long long *raw, double *out, size_t n,
@@ -95,6 +102,10 @@ int run_single_voxel_emission(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_
  * the medium's first such run (synchronously on the context's stream) */
 int ensure_free_map(mcfl_ctx *c, const mcfl_medium *m);
 
+/* run.cpp: the label tiles of the walk kernel, built on a plain medium's
+ * first single-medium run (in the order of the context's stream) */
+int ensure_tiles(mcfl_ctx *c, const mcfl_medium *m);
+
 /* mci.cpp */
 void simulation_geometry(const mcfl_simulation *sim, float *half_x, float *half_y, float *esp, float *g);
 /* Detector-array positions of time-resolved detectors, as the reference
@@ -117,6 +128,8 @@ struct mcfl_medium {
   /* voxel-boundary stepping: label | free radius << 8 per voxel, built on
    * the first such run (mcfl::ensure_free_map) */
   mutable mcfl::DevBuf lab16;
+  /* plain media: the labels in tiles (mcfl::ensure_tiles) */
+  mutable mcfl::DevBuf tiles;
   const float *prop_of(bool emission, bool exact) const {
     return (exact ? (emission ? prop_emi_x : prop_exc_x) : (emission ? prop_emi : prop_exc)).as<float>();
   }

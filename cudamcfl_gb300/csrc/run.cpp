@@ -249,6 +249,14 @@ void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool em
   u.lab16 = exact ? m->lab16.as<uint16_t>() : nullptr;
   u.n_labels = (uint32_t)m->n_bulks + 2u;
   L.plain = m->plain[emission] ? 1u : 0u;
+  if (m->tiles.p) {
+    u.tiles = m->tiles.as<uint8_t>();
+    u.tile_y = 16u * (uint32_t)(m->nx + 1) - 16u;
+    u.tile_z = 16u * (uint32_t)(m->nx + 1) * (uint32_t)(m->ny / 4 + 1) - 4u;
+    u.tile_bytes = (uint32_t)m->tiles.bytes;
+  } else {
+    L.plain = 0; /* no tiles (ensure_tiles was not called): the transport kernel */
+  }
   L.w_event = m->w_event[emission];
   u.fhd = fhd;
   u.hx = m->hx;
@@ -289,6 +297,22 @@ int mcfl::ensure_free_map(mcfl_ctx *c, const mcfl_medium *m) {
   return MCFL_OK;
 }
 
+/* The walk kernel's label tiles, built on a plain medium's first
+ * single-medium run (before any recorded graph uses them). */
+int mcfl::ensure_tiles(mcfl_ctx *c, const mcfl_medium *m) {
+  if (m->tiles.p || !(m->plain[0] || m->plain[1])) return MCFL_OK;
+  const size_t n = (size_t)tile_bytes_of(m->nx, m->ny, m->nz);
+  MCFL_CUDA_TRY(m->tiles.reserve(n));
+  const cudaError_t e = mcfl_launch_tiles(m->labels.as<uint8_t>(), m->nx, m->ny, m->nz, m->total,
+                                          m->tiles.as<uint8_t>(), (uint32_t)n, c->stream);
+  if (e != cudaSuccess) {
+    m->tiles.release();
+    return cuda_fail(e, "label tiles");
+  }
+  ++c->launches;
+  return MCFL_OK;
+}
+
 /* ------------------------------------------------------------------ run */
 
 extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *run, mcfl_run_out *out) {
@@ -301,6 +325,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   cudaGetLastError();
   if (run->exact_stepping && (rc = ensure_free_map(c, m)) != MCFL_OK) return rc;
+  if (!run->exact_stepping && (rc = ensure_tiles(c, m)) != MCFL_OK) return rc;
   cudaStream_t s = c->stream;
   const size_t xy = (size_t)det.nx + (size_t)det.nx * det.ny;
   const size_t nv = m->total;
@@ -546,6 +571,11 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
   }
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   cudaGetLastError();
+  if (!exact)
+    for (int i = 0; i < n; ++i) {
+      const int rct = uniform || schedule == MCFL_SCHEDULE_PLAIN ? ensure_tiles(c, media[i]) : MCFL_OK;
+      if (rct != MCFL_OK) return rct;
+    }
   cudaStream_t s = c->stream;
   const size_t xy = (size_t)det.nx + (size_t)det.nx * det.ny;
   const size_t N = (size_t)n;
@@ -843,6 +873,9 @@ int mcfl::run_single_voxel_emission(mcfl_ctx *c, const mcfl_medium *m, const mcf
   if (run->exact_stepping) {
     const int rcm = ensure_free_map(c, m);
     if (rcm != MCFL_OK) return rcm;
+  } else {
+    const int rct = ensure_tiles(c, m);
+    if (rct != MCFL_OK) return rct;
   }
   MCFL_CUDA_TRY(c->R128.reserve(xy * 16));
   MCFL_CUDA_TRY(c->T128.reserve(xy * 16));

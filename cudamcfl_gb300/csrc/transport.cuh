@@ -1615,7 +1615,7 @@ extern "C" cudaError_t MCFL_LAUNCHER(const McflLaunch *L, int grid, int block, c
 #if !MCFL_F64
   if (walk) {
     const bool timed = v == 3 || v == -2;
-    cfg.dynamicSmemBytes = walk_dynamic(v >= 0, timed, no_phd, block, L->med.n_labels);
+    cfg.dynamicSmemBytes = walk_dynamic(v >= 0, timed, block, L->med.n_labels);
     int dev = 0, max_sm = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -41,13 +41,13 @@ constexpr uint32_t kTailWarps = 2u;    /* warps a block keeps while it has photo
 constexpr uint32_t kSpreadWarps = 12u; /* warps of an SM that a run of few photons is spread over */
 constexpr uint32_t kMixedPool = 64u;   /* photons that move at one meeting, mixed media */
 
-/* Photons set up ahead per warp: rows of kN entries in shared memory.  A
- * direction of their own, a weight and a source index are kept only where
- * emitting voxels can be the source. */
-template <bool kDirs>
+/* Photons set up ahead per warp: rows of kN entries in shared memory (reals:
+ * position, direction, -log of the next step draw; words: stream state,
+ * multiplier, label and kQueuePassed, job, weight, source entry). */
+constexpr uint32_t kQueuePassed = 0x100u; /* the photon has made its first pass */
 struct WalkQueue {
-  static constexpr int kN = kDirs ? 16 : 32;
-  static constexpr int kReals = kDirs ? 7 : 3, kWords = kDirs ? 7 : 5;
+  static constexpr int kN = 16;
+  static constexpr int kReals = 7, kWords = 7;
   static constexpr size_t kBytes = (size_t)kN * (kReals * sizeof(real) + kWords * 4);
   real *f;
   uint32_t *u;
@@ -185,6 +185,9 @@ __device__ __forceinline__ uint32_t walk_voxel(const Med &m, real x, real y, rea
   return min(i, m.total - 1u);
 }
 
+/* The media above and below the slab (labels 0 and last). */
+__device__ __forceinline__ bool walk_outside(uint32_t label, uint32_t last) { return label - 1u >= last - 1u; }
+
 /* move_to_first_boundary() out of line: none of its registers in the kernel's
  * loop (in a plain medium only photons of a source below the slab take it). */
 struct GlassEnd {
@@ -198,17 +201,28 @@ __device__ __noinline__ GlassEnd walk_glass(Photon p, Med m, real max_s) {
   return GlassEnd{p.x, p.y, p.z, label, p.tof};
 }
 
+/* What a warp keeps between its events (all lanes write the same values). */
+struct WalkWarp {
+  unsigned long long seen; /* single medium: the last ticket number seen */
+  uint32_t q_head, q_cnt;  /* single medium: what is left in the warp's queue */
+  /* passes the warp makes before it looks up: a bound below what any of its
+   * photons may still make before the pass cap, and what is left until the
+   * next meeting (the launch's end) or the next look at a slice's end; the
+   * smaller of the two at the last entry into the loop */
+  uint32_t cap_left, period_left, common;
+  uint32_t it; /* slices: passes of the warp */
+};
+
 /* A photon's state while it moves between warps: 7 real rows, then words. */
 constexpr int kPoolReals = 7;
 __host__ __device__ constexpr size_t walk_pool_entry(bool time) { return kPoolReals * sizeof(real) + (time ? 10 : 8) * 4; }
 
 /* Shared memory of a block: static (per-thread words) and dynamic (label
  * records and queues, or the mixed-media pool). */
-constexpr size_t walk_static(int threads) { return (size_t)threads * (5 * 4 + 8) + 64; }
-static size_t walk_dynamic(bool uniform, bool time, bool no_phd, int block, uint32_t n_labels) {
+constexpr size_t walk_static(int threads) { return (size_t)threads * (4 * 4 + 8) + (size_t)threads * 2; }
+static size_t walk_dynamic(bool uniform, bool time, int block, uint32_t n_labels) {
   if (!uniform) return kMixedPool * walk_pool_entry(time);
-  const size_t queue = no_phd && !time ? WalkQueue<true>::kBytes : WalkQueue<false>::kBytes;
-  return (size_t)n_labels * 2 * sizeof(real4) + (size_t)(block / 32) * queue;
+  return (size_t)n_labels * 2 * sizeof(real4) + (size_t)(block / 32) * WalkQueue::kBytes;
 }
 
 /* kUniform: the medium comes from the launch parameters and the label records
@@ -219,8 +233,15 @@ template <bool kUniform, bool kTime, bool kNoPhd, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunch L) {
   constexpr bool kDirs = kNoPhd && !kTime; /* only these launches have emitting voxels */
   constexpr bool kPhd = kUniform && !kTime && !kNoPhd; /* such a launch always tallies it */
+  /* After a pass with decisions in which no photon ended, back to the common
+   * passes at once (true) or by way of the warp's bookkeeping.  Measured:
+   * 1999 strict-math photons 8.8 against 10.3 ms (excitation), served
+   * requests 40.7 against 41.2 ms; but 20011 fast photons 2.8 against 1.8 ms
+   * and 30 beams in one launch 30.2 against 28.5 ms, where the compiler keeps
+   * less of the common pass's state in registers. */
+  constexpr bool kStay = MCFL_EXACT_MATH || !kUniform;
   constexpr bool kSplit = kUniform && kThreads == 128;
-  using Queue = WalkQueue<kDirs>;
+  using Queue = WalkQueue;
   extern __shared__ __align__(16) unsigned char s_mem[];
   real4 *s_lab = reinterpret_cast<real4 *>(s_mem);
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
@@ -233,13 +254,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   const uint32_t pool_size =
       kUniform ? (uint32_t)((n_warps * Queue::kBytes) / walk_pool_entry(kTime)) : kMixedPool;
   uint32_t *pool_u = reinterpret_cast<uint32_t *>(pool_f + kPoolReals * pool_size);
-  /* per lane: the job, the passes of the photon, and of the job since the
-   * last flush the photons ended, their passes and the weight absorbed */
-  __shared__ uint32_t s_job[kThreads], s_pst[kThreads], s_done[kThreads], s_steps[kThreads];
+  /* per lane: the job, and of the job since the last flush the photons
+   * ended, their passes and the weight absorbed */
+  __shared__ uint32_t s_job[kThreads], s_done[kThreads], s_steps[kThreads];
   __shared__ unsigned long long s_absorbed[kThreads];
   __shared__ uint32_t s_src[kDirs ? kThreads : 1];
   __shared__ uint32_t s_live[kThreads / 32];
-  uint32_t &job = s_job[threadIdx.x], &pst = s_pst[threadIdx.x], &done = s_done[threadIdx.x];
+  __shared__ WalkWarp s_warp[kThreads / 32];
+  volatile WalkWarp &w = s_warp[warp];
+  uint32_t &job = s_job[threadIdx.x], &done = s_done[threadIdx.x];
   uint32_t &steps = s_steps[threadIdx.x], &src_idx = s_src[kDirs ? threadIdx.x : 0];
   unsigned long long &absorbed = s_absorbed[threadIdx.x];
   job = 0xffffffffu;
@@ -279,7 +302,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   };
 
   const uint32_t w_event = L.w_event, pst_event = L.step_cap - 1u;
-  const uint64_t ticket_end = L.ticket_end_dev ? *L.ticket_end_dev : L.ticket_end;
+  const uint8_t *tiles = nullptr;
+  uint32_t tile_y = 0, tile_z = 0, tile_last = 0;
+  if (kUniform) {
+    tiles = L.med.tiles;
+    tile_y = L.med.tile_y;
+    tile_z = L.med.tile_z;
+    tile_last = L.med.tile_bytes - 1u;
+  }
+  auto ticket_end_of = [&]() -> uint64_t { return L.ticket_end_dev ? __ldg(L.ticket_end_dev) : L.ticket_end; };
   bool alive = false;
   /* mixed media: the warp's ticket queue; which queues it found exhausted
    * (warp-uniform; a missing second queue counts as exhausted) */
@@ -287,20 +318,19 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   const uint32_t period = L.express_period ? L.express_period : 4u;
   uint32_t tq = two_queues ? (((uint32_t)(gtid >> 5) % period) != 0u ? 1u : 0u) : 0u;
   bool ex0 = false, ex1 = !two_queues;
-  /* single medium: what is left in the warp's queue, the last ticket number
-   * seen, and whether the first photons are still to be drawn */
-  uint32_t q_head = 0, q_cnt = 0;
-  uint64_t seen = 0;
-  bool first = true;
+  bool first = true; /* the first photons are still to be drawn */
   bool tail = false; /* the launch's end: all tickets drawn */
-  /* passes the warp makes before it looks up: a bound below what any of its
-   * photons may still make before the pass cap, and what is left until the
-   * next meeting (the launch's end) or the next look at a slice's end */
-  uint32_t cap_left = pst_event, period_left = 0u;
-  uint32_t it = 0; /* slices: passes of the warp */
+  w.seen = 0;
+  w.q_head = 0;
+  w.q_cnt = 0;
+  w.cap_left = pst_event;
+  w.period_left = 0;
+  w.it = 0;
+  __syncwarp();
 
   real nl = MCFL_C(1.0);     /* -log of the pass's step draw */
   real mutr = MCFL_C(0.0);   /* 1/mu_t of the photon's label */
+  uint32_t pst = 0;          /* the photon's passes */
   uint32_t pst0 = 0;         /* slices: passes before this one */
   uint64_t k = 0;
   auto job_of = [&]() -> const McflJob * { return &L.jobs[job]; };
@@ -346,11 +376,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
       enter_label();
       nl = next_depth();
     }
-    cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+    w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+    __syncwarp();
   }
 
   for (;;) {
-    if (sliced && period_left == 0u) {
+    if (sliced && w.period_left == 0u) {
+      const uint32_t it = w.it;
       if (L.max_iters && it >= L.max_iters) break;
       /* a served slice ends when its time is up or its stop flag is raised
        * (a request arrived, or one finished); lane 0 reads the clock and the
@@ -362,17 +394,21 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
                  (L.stop_flag && *(volatile const unsigned int *)L.stop_flag != 0u);
         if (__shfl_sync(kFull, stop, 0)) break;
       }
-      period_left = L.max_iters ? min(64u, L.max_iters - it) : 64u;
+      __syncwarp();
+      w.period_left = L.max_iters ? min(64u, L.max_iters - it) : 64u;
+      __syncwarp();
     }
     unsigned dead = __ballot_sync(kFull, !alive);
-    if (!sliced && ex0 && ex1 && q_cnt == 0 && (tail || dead)) {
-      if (!tail) period_left = 0u;
+    if (!sliced && ex0 && ex1 && (tail || dead) && w.q_cnt == 0) {
+      const bool meet = !tail || w.period_left == 0u || dead == kFull;
       tail = true;
-      if (period_left == 0u || dead == kFull) {
-        /* ---- a meeting: the block's photons move together.  The first
-         * `keep` warps in an order that starts at another warp in each block
-         * of an SM (so that the schedulers share them) hold up to `per`
-         * photons; the other warps' photons go to their free lanes. ---- */
+      if (meet) {
+        /* ---- a meeting: the block's photons are shared out evenly among
+         * its first `keep` warps, in an order that starts at another warp in
+         * each block of an SM (so that the schedulers share them).  Enough
+         * warps to hold them, and kTailWarps while there are photons for
+         * these: a lane waits for the events of its warp's other lanes, so
+         * few lanes per warp are as good as the issue slots allow. ---- */
         const unsigned start = L.sm_count ? (blockIdx.x / L.sm_count) % n_warps : 0u;
         const unsigned order = (warp + n_warps - start) % n_warps;
         if (lane == 0) s_live[order] = 32u - (uint32_t)__popc(dead);
@@ -384,19 +420,20 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         const uint32_t per = (total + keep - 1u) / keep;
         uint32_t give = 0, give_at = 0, room = 0, take_at = 0;
         for (unsigned i = 0; i < n_warps; ++i) {
-          const uint32_t l = s_live[i], free_i = l < per ? per - l : 0u;
-          if (i < keep) {
-            if (i < order) take_at += free_i;
-            room += free_i;
-          } else {
-            if (i < order) give_at += l;
-            give += l;
+          const uint32_t l = s_live[i], most = i < keep ? per : 0u;
+          const uint32_t over = l > most ? l - most : 0u, under = l < most ? most - l : 0u;
+          if (i < order) {
+            give_at += over;
+            take_at += under;
           }
+          give += over;
+          room += under;
         }
         give = min(min(give, room), pool_size);
-        const uint32_t rank = __popc((order < keep ? dead : ~dead) & ((1u << lane) - 1u));
-        if (order >= keep && alive && give_at + rank < give) {
-          const uint32_t e = give_at + rank;
+        const uint32_t mine = s_live[order], most = order < keep ? per : 0u;
+        const uint32_t above = __popc(~dead & ((1u << lane) - 1u)), free_above = __popc(dead & ((1u << lane) - 1u));
+        if (alive && above >= most && give_at + (above - most) < give) {
+          const uint32_t e = give_at + (above - most);
           pool_f[e] = p.x;
           pool_f[pool_size + e] = p.y;
           pool_f[2 * pool_size + e] = p.z;
@@ -419,8 +456,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
           alive = false;
         }
         __syncthreads();
-        if (order < keep && !alive && rank + s_live[order] < per && take_at + rank < give) {
-          const uint32_t e = take_at + rank;
+        if ((dead >> lane & 1u) && mine + free_above < most && take_at + free_above < give) {
+          const uint32_t e = take_at + free_above;
           const uint32_t j = pool_u[5 * pool_size + e];
           if (j != job) {
             flush_stats();
@@ -445,12 +482,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
           alive = true;
         }
         __syncthreads();
-        period_left = kTailPasses;
-        cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+        w.period_left = kTailPasses;
+        w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+        __syncwarp();
       }
     } else if (dead && ((uint32_t)__popc(dead) >= L.relaunch_min || dead == kFull)) {
       if constexpr (kUniform) {
-        uint32_t want = __popc(dead);
+        uint32_t want = __popc(dead), q_head = w.q_head, q_cnt = w.q_cnt;
+        const uint64_t ticket_end = ticket_end_of();
         if (first && L.sm_count) {
           /* few photons: as many per warp as spread them over kSpreadWarps
            * warps of each SM (they share its issue slots either way; fewer
@@ -465,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
             __syncwarp();
             /* set up the photons wanted now, and ahead of them half of the
              * warp's share of what is left */
-            const uint64_t left = ticket_end > seen ? ticket_end - seen : 0ull;
+            const uint64_t seen = w.seen, left = ticket_end > seen ? ticket_end - seen : 0ull;
             const uint32_t warps = gridDim.x * n_warps;
             uint32_t fill = left >= (uint64_t)warps * (2 * Queue::kN) ? (uint32_t)Queue::kN
                                                                      : (uint32_t)left / (2u * warps);
@@ -473,7 +512,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
             unsigned long long base = 0ull;
             if (lane == 0) base = atomicAdd(L.ticket_counter, (unsigned long long)fill);
             base = __shfl_sync(kFull, base, 0);
-            seen = base + fill;
+            w.seen = base + fill;
             const uint32_t got =
                 base >= ticket_end ? 0u : (uint32_t)min((unsigned long long)fill, (unsigned long long)ticket_end - base);
             if (got < fill) ex0 = true;
@@ -489,22 +528,46 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
                 uint32_t src = 0;
                 launch_photon<0, kDirs>(J, m, kk, L.mult, f, fr, src);
                 real fnl = MCFL_C(1.0);
-                if (s_lab[2 * f.label].x != walk_no_step()) fnl = walk_depth(fr);
+                uint32_t passed = 0u;
+                if (s_lab[2 * f.label].x != walk_no_step()) {
+                  fnl = walk_depth(fr);
+                  /* a beam starts along the z axis, where the deflection has
+                   * a form of its own: its first pass, when it is common
+                   * otherwise, is made here, by all lanes */
+                  const real fs = fp_mul(fnl, s_lab[2 * f.label].x), fz = fp_fma(fs, f.dz, f.z);
+                  const real fq = fp_one_minus_sq(f.dz);
+                  if (!kTime && !(fq > MCFL_C(0.0)) && fminf(fz, fs) > MCFL_C(0.0) && fz < m.esp && f.weight > w_event &&
+                      pst_event > 0u) {
+                    const uint32_t w0 = f.weight;
+                    f.x = fp_fma(f.dx, fs, f.x);
+                    f.y = fp_fma(f.dy, fs, f.y);
+                    f.z = fz;
+                    const bool in = MCFL_FABS(f.x) < m.hx && MCFL_FABS(f.y) < m.hy;
+                    const uint32_t v = walk_voxel(m, f.x, f.y, f.z);
+                    f.label = in ? (uint32_t)m.labels[v] : 1u;
+                    if (kPhd && in) atomicAdd(&m.fhd[v], (unsigned long long)w0);
+                    real u_hg, cosp, sinp;
+                    walk_draw(fr, u_hg, cosp, sinp);
+                    const Rec c = rec_of_label(f.label);
+                    f.weight -= MCFL_R2U_RU(fp_mul(c.a.y, MCFL_U2R_RN(w0)));
+                    walk_spin<true, kSplit>(f, c, u_hg, cosp, sinp, fq);
+                    fnl = walk_depth(fr);
+                    passed = kQueuePassed;
+                  }
+                }
                 queue.f[0 * Queue::kN + lane] = f.x;
                 queue.f[1 * Queue::kN + lane] = f.y;
-                queue.f[2 * Queue::kN + lane] = fnl;
+                queue.f[2 * Queue::kN + lane] = f.z;
+                queue.f[3 * Queue::kN + lane] = f.dx;
+                queue.f[4 * Queue::kN + lane] = f.dy;
+                queue.f[5 * Queue::kN + lane] = f.dz;
+                queue.f[6 * Queue::kN + lane] = fnl;
                 queue.u[0 * Queue::kN + lane] = (uint32_t)fr.x;
                 queue.u[1 * Queue::kN + lane] = (uint32_t)(fr.x >> 32);
                 queue.u[2 * Queue::kN + lane] = fr.a;
-                queue.u[3 * Queue::kN + lane] = f.label;
-                if constexpr (kDirs) {
-                  queue.f[3 * Queue::kN + lane] = f.z;
-                  queue.f[4 * Queue::kN + lane] = f.dx;
-                  queue.f[5 * Queue::kN + lane] = f.dy;
-                  queue.f[6 * Queue::kN + lane] = f.dz;
-                  queue.u[5 * Queue::kN + lane] = f.weight;
-                  queue.u[6 * Queue::kN + lane] = src;
-                }
+                queue.u[3 * Queue::kN + lane] = f.label | passed;
+                queue.u[5 * Queue::kN + lane] = f.weight;
+                queue.u[6 * Queue::kN + lane] = src;
               }
               queue.u[4 * Queue::kN + lane] = j;
             }
@@ -525,28 +588,25 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
               }
               p.x = queue.f[0 * Queue::kN + e];
               p.y = queue.f[1 * Queue::kN + e];
-              nl = queue.f[2 * Queue::kN + e];
+              p.z = queue.f[2 * Queue::kN + e];
+              p.dx = queue.f[3 * Queue::kN + e];
+              p.dy = queue.f[4 * Queue::kN + e];
+              p.dz = queue.f[5 * Queue::kN + e];
+              nl = queue.f[6 * Queue::kN + e];
               r.x = ((uint64_t)queue.u[1 * Queue::kN + e] << 32) | queue.u[0 * Queue::kN + e];
               r.a = queue.u[2 * Queue::kN + e];
-              p.label = queue.u[3 * Queue::kN + e];
-              if constexpr (kDirs) {
-                p.z = queue.f[3 * Queue::kN + e];
-                p.dx = queue.f[4 * Queue::kN + e];
-                p.dy = queue.f[5 * Queue::kN + e];
-                p.dz = queue.f[6 * Queue::kN + e];
-                p.weight = queue.u[5 * Queue::kN + e];
-                src_idx = queue.u[6 * Queue::kN + e];
-              } else {
-                p.z = __ldg(&job_of()->sz);
-                p.dx = MCFL_C(0.0);
-                p.dy = MCFL_C(0.0);
-                p.dz = MCFL_C(1.0);
-                p.weight = __ldg(&job_of()->start_weight);
-              }
+              const uint32_t lp = queue.u[3 * Queue::kN + e];
+              p.label = lp & 0xffu;
+              p.weight = queue.u[5 * Queue::kN + e];
+              if constexpr (kDirs) src_idx = queue.u[6 * Queue::kN + e];
               p.tof = 0;
               enter_label();
-              pst = 0;
-              absorbed += p.weight;
+              pst = lp / kQueuePassed;
+              /* the weight it started with: only emitting voxels' photons
+               * have another weight than the job's */
+              absorbed += !(lp & kQueuePassed) ? p.weight : kDirs && __ldg(&job_of()->src_kind) == MCFL_SRC_VOXELS
+                                                               ? 0xFFFFFFFFu
+                                                               : __ldg(&job_of()->start_weight);
               alive = true;
             }
           }
@@ -555,13 +615,17 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
           want -= take;
           dead = __ballot_sync(kFull, !alive);
         }
+        __syncwarp();
+        w.q_head = q_head;
+        w.q_cnt = q_cnt;
+        __syncwarp();
       } else {
         /* mixed media: the free lanes set up their own photons */
         const bool need = !alive && !(ex0 && ex1);
         const unsigned nm = __ballot_sync(kFull, need);
         if (nm) {
           unsigned long long *ctr = L.ticket_counter;
-          uint64_t end = ticket_end;
+          uint64_t end = ticket_end_of();
           if (tq ? ex1 : ex0) tq ^= 1u;
           if (tq) {
             ctr = L.ticket_counter2;
@@ -612,22 +676,20 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
     }
     uint32_t made = 0;
     if (alive) {
-      const uint32_t common = (sliced || tail) ? min(cap_left, period_left) : cap_left;
-      uint32_t left = common;
+      uint32_t left = w.cap_left;
+      if (sliced || tail) left = min(left, w.period_left);
+      w.common = left;
       real zn, xn, yn, s, q;
       bool inside, special;
       uint32_t vi, g;
       Rec c;
       real u_hg, cosp, sinp;
-      const real n_in = kTime ? rec_of_label(1u).b.w : MCFL_C(0.0); /* every label's index */
-      auto commit = [&]() {
-        p.x = xn;
-        p.y = yn;
-        p.z = zn;
-        p.label = inside ? g : 1u;
-        if constexpr (kTime) p.tof += tof_fs(fp_mul(s, n_in));
-        if ((kPhd || (!kNoPhd && m.fhd)) && inside) atomicAdd(&m.fhd[vi], (unsigned long long)p.weight);
+      /* the hitting density at a point that is not a common pass's end */
+      auto tally_at = [&](real x, real y, real z, uint32_t w) {
+        if ((kPhd || (!kNoPhd && m.fhd)) && MCFL_FABS(x) < m.hx && MCFL_FABS(y) < m.hy && z < m.esp)
+          atomicAdd(&m.fhd[walk_voxel(m, x, y, z)], (unsigned long long)w);
       };
+      for (;;) { /* kStay: until a photon ends or the warp has to look up */
       /* ---- common passes, until one is special for some lane ---- */
       for (;;) {
         s = fp_mul(nl, mutr);
@@ -635,17 +697,29 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         xn = fp_fma(p.dx, s, p.x);
         yn = fp_fma(p.dy, s, p.y);
         inside = MCFL_FABS(xn) < m.hx && MCFL_FABS(yn) < m.hy;
-        vi = walk_voxel(m, xn, yn, zn);
+        const uint32_t ix = MCFL_R2U_RZ(fp_mul(fp_add(xn, m.hx), m.gx)),
+                       iy = MCFL_R2U_RZ(fp_mul(fp_add(yn, m.hy), m.gy)), iz = MCFL_R2U_RZ(fp_mul(zn, m.gz));
+        const uint8_t *at;
+        if (!kUniform || kTime || !kNoPhd) vi = min(ix + m.nx * (iy + m.ny * iz), m.total - 1u);
+        if (kUniform)
+          at = tiles + min(ix * 16u + (iy * 4u + (iz + (iy >> 2) * tile_y + (iz >> 2) * tile_z)), tile_last);
+        else
+          at = m.labels + vi;
         /* the end point's label, kept in L1 ahead of other lines (evict-last
          * hint) */
-        asm("ld.global.nc.L1::evict_last.u8 %0, [%1];" : "=r"(g) : "l"(m.labels + vi));
+        asm("ld.global.nc.L1::evict_last.u8 %0, [%1];" : "=r"(g) : "l"(at));
         q = fp_one_minus_sq(p.dz);
         special = !(fminf(fminf(zn, s), q) > MCFL_C(0.0)) || !(zn < m.esp) || p.weight <= w_event || left == 0u;
         if (__any_sync(live, special)) break;
         --left;
         walk_draw(r, u_hg, cosp, sinp);
-        c = rec_of_label(inside ? g : 1u);
-        commit();
+        p.label = inside ? g : 1u;
+        c = rec_of_label(p.label);
+        p.x = xn;
+        p.y = yn;
+        p.z = zn;
+        if constexpr (kTime) p.tof += tof_fs(fp_mul(s, c.b.w)); /* every label has this index */
+        if ((kPhd || (!kNoPhd && m.fhd)) && inside) atomicAdd(&m.fhd[vi], (unsigned long long)p.weight);
         p.weight -= MCFL_R2U_RU(fp_mul(c.a.y, MCFL_U2R_RN(p.weight)));
         walk_spin<false, kSplit>(p, c, u_hg, cosp, sinp, q);
         mutr = c.a.x;
@@ -655,20 +729,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
       /* ---- one pass with its decisions: the special lanes run the
        * reference's sequence up to the deflection, which all lanes then make
        * together ---- */
-      made = common - left + 1u;
-      const uint32_t passes = pst + made;
-      pst = passes;
       inside = inside && zn < m.esp;
-      special = !(fminf(fminf(zn, s), q) > MCFL_C(0.0)) || !(zn < m.esp) || p.weight <= w_event || passes > pst_event;
+      special = !(fminf(fminf(zn, s), q) > MCFL_C(0.0)) || !(zn < m.esp) || p.weight <= w_event || left == 0u;
       bool spin_now = true;
+      const uint32_t lab = inside ? g : 1u;
       if (special) {
-        const uint32_t lab = inside ? g : 1u;
-        const Rec c_old = load_rec(m, p.label);
-        const real n_old = c_old.b.w;
-        const bool glass = !(c_old.a.x != FLT_MAX); /* a source below the slab */
-        const bool clip = zn < MCFL_C(0.0) || zn > m.esp;
-        const uint32_t phd_w = p.weight; /* before an exit takes it */
-        uint32_t phd_idx = 0xffffffffu, new_bulk = lab;
+        const real n_old = rec_of_label(p.label).b.w;
+        const bool glass = mutr == walk_no_step(); /* a source below the slab */
+        const uint32_t w0 = p.weight; /* before an exit takes it */
+        uint32_t new_bulk = lab;
+        bool stays = s > MCFL_C(0.0) && lab == p.label;
         if (glass) { /* scattering-free: it drew no step length */
           s = MCFL_C(100.0);
           const GlassEnd e = walk_glass<kTime>(p, m, s);
@@ -677,8 +747,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
           p.z = e.z;
           if constexpr (kTime) p.tof = e.tof;
           new_bulk = e.label;
+          stays = false;
         } else {
-          if (clip) { /* the step reaches a slab face */
+          if (zn < MCFL_C(0.0) || zn > m.esp) { /* the step reaches a slab face */
             new_bulk = p.label;
             if (zn < MCFL_C(0.0)) {
               new_bulk = 0;
@@ -691,23 +762,17 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
             xn = fp_fma(p.dx, s, p.x);
             yn = fp_fma(p.dy, s, p.y);
             zn = fp_fma(p.dz, s, p.z);
-          } else if (inside) {
-            phd_idx = vi;
+            stays = false;
           }
           p.x = xn;
           p.y = yn;
           p.z = zn;
           if constexpr (kTime) p.tof += tof_fs(fp_mul(s, n_old));
         }
-        const bool stays = !glass && !clip && s > MCFL_C(0.0) && lab == p.label;
-        if (new_bulk != p.label && walk_reflect(p, n_old, load_rec(m, new_bulk).b.w, r)) p.label = new_bulk;
-        if ((kPhd || (!kNoPhd && m.fhd)) &&
-            (phd_idx != 0xffffffffu || (MCFL_FABS(p.x) < m.hx && MCFL_FABS(p.y) < m.hy && p.z < m.esp))) {
-          if (phd_idx == 0xffffffffu) phd_idx = walk_voxel(m, p.x, p.y, p.z);
-          atomicAdd(&m.fhd[phd_idx], (unsigned long long)phd_w);
-        }
+        if (new_bulk != p.label && walk_reflect(p, n_old, rec_of_label(new_bulk).b.w, r)) p.label = new_bulk;
+        tally_at(p.x, p.y, p.z, w0);
         spin_now = s > MCFL_C(0.0);
-        if (!stays && (p.label == 0u || p.label == m.last)) {
+        if (!stays && walk_outside(p.label, m.last)) {
           const bool top = p.label == 0u;
           tally_exit(job_of(), p.x, p.y, p.weight, top, kDirs ? src_idx : 0u);
           if constexpr (kTime) tally_time(job_of(), p.x, p.y, p.weight, p.tof, top);
@@ -718,7 +783,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         }
         q = fp_one_minus_sq(p.dz);
       } else {
-        commit();
+        p.x = xn;
+        p.y = yn;
+        p.z = zn;
+        p.label = lab;
+        if constexpr (kTime) p.tof += tof_fs(fp_mul(s, rec_of_label(lab).b.w));
+        if ((kPhd || (!kNoPhd && m.fhd)) && inside) atomicAdd(&m.fhd[vi], (unsigned long long)p.weight);
       }
       if (spin_now) {
         walk_draw(r, u_hg, cosp, sinp);
@@ -744,6 +814,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
             alive = false;
           }
         }
+        const uint32_t passes = pst + (w.common - left) + 1u;
         if (alive && passes >= L.step_cap) {
           ev_add(MCFL_ST_CAPPED, 1ull);
           absorbed -= p.weight;
@@ -767,15 +838,23 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         }
       }
       if (alive) nl = next_depth();
+      if (!kStay || left == 0u || __any_sync(live, !alive)) break;
+      --left;
+      }
+      made = w.common - left + 1u;
+      pst += made;
     }
     /* lanes without a photon did not count the passes */
     made = __shfl_sync(kFull, made, __ffs(live) - 1);
-    if (sliced || tail) period_left -= min(made, period_left);
-    if (sliced) it += made;
-    if (made > cap_left) /* the bound is used up */
-      cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
-    else
-      cap_left -= made;
+    const uint32_t cap_left = w.cap_left, period_left = w.period_left, it = w.it;
+    /* past the bound, it is taken anew */
+    const uint32_t cap_now = made > cap_left ? __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event)
+                                             : cap_left - made;
+    __syncwarp();
+    w.cap_left = cap_now;
+    if (sliced || tail) w.period_left = period_left - min(made, period_left);
+    if (sliced) w.it = it + made;
+    __syncwarp();
   }
   if (alive) {
     steps += pst - pst0; /* passes of the photon parked by this slice */
