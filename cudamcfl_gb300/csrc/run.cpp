@@ -14,6 +14,8 @@
  * schedules give bit-identical tallies; only their speed differs.
  */
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstring>
@@ -113,6 +115,26 @@ int check_run(const mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *run)
     if (!inside) return fail(MCFL_E_ARG, "layered medium: the source z lies in no slab");
   }
   return MCFL_OK;
+}
+
+/* Brings the pages of an output buffer in while the GPU computes: a copy into
+ * pages that the host has not written yet faults on the GPU side, about 50 us
+ * for each page (26 ms for a fresh 32 MB array, 0.2 ms for a touched one).
+ * The contents stay as they are.  Each page is faulted for writing at once; a
+ * read before the write would map the zero page first and have its mapping
+ * taken back from the GPU again (20 us for each page). */
+void touch_pages(void *p, size_t bytes) {
+  if (!p || !bytes) return;
+  const long n = sysconf(_SC_PAGESIZE);
+  const uintptr_t page = n > 0 ? (uintptr_t)n : 4096u;
+  const uintptr_t lo = (uintptr_t)p & ~(page - 1), hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
+#ifdef MADV_POPULATE_WRITE
+  if (madvise((void *)lo, hi - lo, MADV_POPULATE_WRITE) == 0) return;
+#else
+  (void)hi;
+#endif
+  for (uintptr_t a = lo < (uintptr_t)p ? (uintptr_t)p : lo; a < (uintptr_t)p + bytes; a = (a & ~(page - 1)) + page)
+    __atomic_fetch_or((unsigned char *)a, 0, __ATOMIC_RELAXED);
 }
 
 cudaError_t ensure_pinned(mcfl_ctx *c, size_t jobs, size_t outs) {
@@ -473,6 +495,21 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
   /* FP64 normalisation of the requested images on the GPU */
   std::vector<std::pair<double *, std::pair<double *, size_t>>> pend;
   if (out) {
+    touch_pages(out->R, xy * 8);
+    touch_pages(out->T, xy * 8);
+    touch_pages(out->Rd, xy * 8);
+    touch_pages(out->Tt, xy * 8);
+    if (fluence) {
+      touch_pages(out->phd, nv * 8);
+      touch_pages(out->fhd, nv * 8);
+    }
+    if (emission) {
+      touch_pages(out->flR, xy * 8);
+      touch_pages(out->flT, xy * 8);
+      touch_pages(out->flR128, xy * 16);
+      touch_pages(out->flT128, xy * 16);
+    }
+    if (timed) touch_pages(out->time_xyt, tsize * 8);
     size_t nd = (out->R ? xy : 0) + (out->T ? xy : 0) + (out->phd && fluence ? nv : 0) +
                 (emission ? (out->flR ? xy : 0) + (out->flT ? xy : 0) : 0);
     if (nd) MCFL_CUDA_TRY(c->outd.reserve(nd * 8));
@@ -680,6 +717,14 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
                  (unsigned long long)c->mixed_code(), c->relaunch, limits.plain, limits.w_event});
     const int rcb = replay(c, &c->graph_batch, &c->graph_batch_key, &c->graph_batch_kernels, key, record);
     if (rcb != MCFL_OK) return rcb;
+    if (outs)
+      for (int i = 0; i < n; ++i) {
+        touch_pages(outs[i].Rd, xy * 8);
+        touch_pages(outs[i].Tt, xy * 8);
+        touch_pages(outs[i].R, xy * 8);
+        touch_pages(outs[i].T, xy * 8);
+        touch_pages(outs[i].time_xyt, (toff[i + 1] - toff[i]) * 8);
+      }
     MCFL_CUDA_TRY(cudaStreamSynchronize(s));
     ms = elapsed_ms(c->ev[0], c->ev[1]);
   } else {
