@@ -730,6 +730,57 @@ __device__ __noinline__ void tally_time(const McflJob *J, real px, real py, uint
 
 } // namespace
 
+/* The launch's end in the transport kernel's single-medium launches: once all
+ * tickets are drawn, the warps of a block meet every kMeetPasses passes and
+ * share their photons out evenly among as few warps as hold them (at least
+ * kMeetWarps while there are photons for these), so that the long-lived
+ * photons do not keep every warp issuing passes for one or two lanes.  The
+ * photons move through kMeetPool entries of shared memory.  Measured in strict
+ * math: 1e6 + 5e5 photons in a medium of several indices 24.4 + 21.6 -> 21.4 +
+ * 19.2 ms; layered, 1e6 photons fast, 7.6 -> 7.15 ms.
+ * Not in the fast build's voxelized kernels: the compiler contracts their
+ * passes another way when code is added, and their results would change. */
+__host__ __device__ constexpr bool meets(bool layered) { return !MCFL_F64 && (MCFL_EXACT_MATH || layered); }
+constexpr uint32_t kMeetPasses = 256u, kMeetWarps = 2u, kMeetPool = 64u;
+/* a run of few photons is spread over this many warps of each SM */
+constexpr uint32_t kFirstWarps = 12u;
+
+struct MovedPhoton {
+  real x, y, z, dx, dy, dz;
+  uint32_t weight, label, rng_lo, rng_hi, rng_a, job, src_idx, pst;
+};
+struct MovedStep { /* voxel-boundary stepping: the pass in progress */
+  real xtau, xox, xoy, xoz, xs0;
+  int ix, iy, iz, xcr, xit;
+  uint32_t flags;
+};
+
+/* Who moves where: warp `order` (of n) gives its photons from the give'th
+ * lane with a photon on to pool entries from give_at, or takes photons into
+ * its free lanes, up to `most` in all, from entry take_at; `moved` entries
+ * are used.  live: the photons of each warp. */
+struct Meeting {
+  uint32_t most, give_at, take_at, moved;
+};
+__device__ __forceinline__ Meeting plan_meeting(const uint32_t *live, unsigned n, unsigned order, uint32_t total,
+                                                uint32_t pool) {
+  const uint32_t keep = min(n, max((total + 31u) >> 5, kMeetWarps)), per = (total + keep - 1u) / keep;
+  Meeting t = {order < keep ? per : 0u, 0u, 0u, 0u};
+  uint32_t give = 0, room = 0;
+  for (unsigned i = 0; i < n; ++i) {
+    const uint32_t l = live[i], most = i < keep ? per : 0u;
+    const uint32_t over = l > most ? l - most : 0u, under = l < most ? most - l : 0u;
+    if (i < order) {
+      t.give_at += over;
+      t.take_at += under;
+    }
+    give += over;
+    room += under;
+  }
+  t.moved = min(min(give, room), pool);
+  return t;
+}
+
 /* One warp-synchronous persistent loop per thread; see the file comment.
  * kUniform: the medium comes from the launch parameters (constant bank)
  * instead of per-lane registers loaded from the job. */
@@ -756,6 +807,14 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
    * medium */
   extern __shared__ __align__(16) unsigned char s_mem[];
   real4 *s_lab = reinterpret_cast<real4 *>(s_mem);
+  /* the launch's end gathered into few warps (see MovedPhoton) */
+  constexpr bool kMeet = kUniform && !kPhdAgg && !kGeneral && !kPhdWarp && meets(kLayered);
+  MovedPhoton *s_moved = reinterpret_cast<MovedPhoton *>(s_mem + lab_bytes(kUniform));
+  MovedStep *s_step = reinterpret_cast<MovedStep *>(s_moved + kMeetPool);
+  __shared__ uint32_t s_live[kMeet ? kThreads / 32 : 1];
+  __shared__ uint64_t s_tof[kMeet && kTime ? kMeetPool : 1];
+  bool tail = false, first = true;
+  uint32_t meet_in = 0;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned tib = threadIdx.x;
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -906,12 +965,90 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
      * of any warp-wide operation inside the pass */
     unsigned live = kFull;
     const unsigned dead = __ballot_sync(kFull, !alive);
-    if (dead) {
+    if (kMeet && (tail || (dead && ex0))) {
+      tail = true;
+      if (meet_in == 0u || dead == kFull) {
+        const unsigned n_warps = blockDim.x >> 5;
+        const unsigned start = L.sm_count ? (blockIdx.x / L.sm_count) % n_warps : 0u;
+        const unsigned order = ((tib >> 5) + n_warps - start) % n_warps;
+        if (lane == 0) s_live[order] = 32u - (uint32_t)__popc(dead);
+        __syncthreads();
+        uint32_t total = 0;
+        for (unsigned i = 0; i < n_warps; ++i) total += s_live[i];
+        if (total == 0u) break;
+        const Meeting t = plan_meeting(s_live, n_warps, order, total, kMeetPool);
+        const uint32_t mine = s_live[order], below = (1u << lane) - 1u;
+        const uint32_t above = __popc(~dead & below), free_above = __popc(dead & below);
+        if (alive && above >= t.most && t.give_at + (above - t.most) < t.moved) {
+          const uint32_t e = t.give_at + (above - t.most);
+          s_moved[e] = MovedPhoton{p.x, p.y, p.z, p.dx, p.dy, p.dz, p.weight, p.label, (uint32_t)r.x,
+                                   (uint32_t)(r.x >> 32), r.a, job, src_idx, pst};
+          if constexpr (kTime) s_tof[e] = p.tof;
+          if constexpr (kExactStep)
+            s_step[e] = MovedStep{xtau, xox, xoy, xoz, xs0, p.ix, p.iy, p.iz, xcr, xit,
+                                  (xmid ? 1u : 0u) | (xbegin ? 2u : 0u)};
+          alive = false;
+        }
+        __syncthreads();
+        if ((dead >> lane & 1u) && mine + free_above < t.most && t.take_at + free_above < t.moved) {
+          const uint32_t e = t.take_at + free_above;
+          const MovedPhoton v = s_moved[e];
+          if (v.job != job) {
+            flush_stats();
+            job = v.job;
+            J = &L.jobs[job];
+          }
+          p.x = v.x;
+          p.y = v.y;
+          p.z = v.z;
+          p.dx = v.dx;
+          p.dy = v.dy;
+          p.dz = v.dz;
+          p.weight = v.weight;
+          p.label = v.label;
+          r.x = ((uint64_t)v.rng_hi << 32) | v.rng_lo;
+          r.a = v.rng_a;
+          src_idx = v.src_idx;
+          pst = v.pst;
+          pst0 = 0;
+          if constexpr (kTime) p.tof = s_tof[e];
+          if constexpr (kExactStep) {
+            const MovedStep w = s_step[e];
+            xtau = w.xtau;
+            xox = w.xox;
+            xoy = w.xoy;
+            xoz = w.xoz;
+            xs0 = w.xs0;
+            p.ix = w.ix;
+            p.iy = w.iy;
+            p.iz = w.iz;
+            xcr = w.xcr;
+            xit = w.xit;
+            xmid = (w.flags & 1u) != 0u;
+            xbegin = (w.flags & 2u) != 0u;
+          }
+          if (kLean) {
+            mutr_c = s_lab[2 * p.label].x;
+            n_c = s_lab[2 * p.label + 1].w;
+          }
+          alive = true;
+        }
+        __syncthreads();
+        meet_in = kMeetPasses;
+      }
+      --meet_in;
+      if (!alive) continue;
+    } else if (dead) {
     /* lanes without a photon draw new ones together once at least
      * relaunch_min of them are free (0 or 1: at once), or every lane is;
      * until then they skip the pass below */
     if ((uint32_t)__popc(dead) >= L.relaunch_min || dead == kFull) {
-    const bool need = !alive && !(ex0 && ex1);
+    bool need = !alive && !(ex0 && ex1);
+    if (kMeet && first && L.sm_count) {
+      const uint64_t spread = (uint64_t)kFirstWarps * L.sm_count;
+      need = need && (uint64_t)lane < (ticket_end + spread - 1u) / spread;
+    }
+    first = false;
     const unsigned nm = __ballot_sync(kFull, need);
     if (nm) {
       unsigned long long *ctr = L.ticket_counter;
@@ -963,7 +1100,7 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
         else ex0 = true;
       }
     }
-    if (__all_sync(kFull, !alive) && ex0 && ex1) break;
+    if (!kMeet && __all_sync(kFull, !alive) && ex0 && ex1) break;
     }
     if constexpr (kPhdWarp) live = __ballot_sync(kFull, alive);
     if (!alive) continue; /* a lane without a photon never runs the pass */
@@ -1561,7 +1698,13 @@ static TransportKernel kernel_of(int variant, int *threads, bool plain = false, 
 }
 
 /* dynamic shared memory of a transport-kernel launch */
-static size_t smem_bytes(bool uniform) { return lab_bytes(uniform) + 16; }
+static size_t smem_bytes(int variant) {
+  const bool stepping = variant == 6 || variant == 10, layered = variant == 4 || variant == 5;
+  const size_t pool = variant >= 0 && variant <= 10 && !(variant >= 7 && variant <= 9) && meets(layered)
+                          ? kMeetPool * (sizeof(MovedPhoton) + (stepping ? sizeof(MovedStep) : 0))
+                          : 0;
+  return lab_bytes(variant >= 0) + 16 + pool;
+}
 
 /* The L1/shared split [%]: just the shared memory that bps blocks need (1 KB
  * per block is reserved by the system), the rest as L1 (the label gather of
@@ -1599,7 +1742,7 @@ extern "C" cudaError_t MCFL_LAUNCHER(const McflLaunch *L, int grid, int block, c
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem_bytes(L->uniform_medium != 0);
+  cfg.dynamicSmemBytes = smem_bytes(v);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   memset(attr, 0, sizeof(attr));
@@ -1644,7 +1787,7 @@ extern "C" cudaError_t MCFL_ATTR_FN(int variant, int *block, int *blocks_per_sm,
   if (e != cudaSuccess) return e;
   if (regs) *regs = a.numRegs;
   if (*block <= 0 || *block > t) *block = t;
-  const size_t smem = smem_bytes(variant >= 0);
+  const size_t smem = smem_bytes(variant);
   /* occupancy with the whole shared memory available */
   e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                            (int)cudaSharedmemCarveoutMaxShared);
