@@ -302,6 +302,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   };
 
   const uint32_t w_event = L.w_event, pst_event = L.step_cap - 1u;
+  /* common passes that any new photon may make: it may have made its first */
+  const uint32_t fresh_left = max(pst_event, 1u) - 1u;
   const uint8_t *tiles = nullptr;
   uint32_t tile_y = 0, tile_z = 0, tile_last = 0;
   if (kUniform) {
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   w.seen = 0;
   w.q_head = 0;
   w.q_cnt = 0;
-  w.cap_left = pst_event;
+  w.cap_left = fresh_left;
   w.period_left = 0;
   w.it = 0;
   __syncwarp();
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
       enter_label();
       nl = next_depth();
     }
-    w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+    w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : fresh_left);
     __syncwarp();
   }
 
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         }
         __syncthreads();
         w.period_left = kTailPasses;
-        w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event);
+        w.cap_left = __reduce_min_sync(kFull, alive ? pst_event - pst : fresh_left);
         __syncwarp();
       }
     } else if (dead && ((uint32_t)__popc(dead) >= L.relaunch_min || dead == kFull)) {
@@ -848,7 +850,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
     made = __shfl_sync(kFull, made, __ffs(live) - 1);
     const uint32_t cap_left = w.cap_left, period_left = w.period_left, it = w.it;
     /* past the bound, it is taken anew */
-    const uint32_t cap_now = made > cap_left ? __reduce_min_sync(kFull, alive ? pst_event - pst : pst_event)
+    const uint32_t cap_now = made > cap_left ? __reduce_min_sync(kFull, alive ? pst_event - pst : fresh_left)
                                              : cap_left - made;
     __syncwarp();
     w.cap_left = cap_now;
