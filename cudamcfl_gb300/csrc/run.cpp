@@ -128,13 +128,7 @@ void touch_pages(void *p, size_t bytes) {
   const long n = sysconf(_SC_PAGESIZE);
   const uintptr_t page = n > 0 ? (uintptr_t)n : 4096u;
   const uintptr_t lo = (uintptr_t)p & ~(page - 1), hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
-#ifdef MADV_POPULATE_WRITE
-  if (madvise((void *)lo, hi - lo, MADV_POPULATE_WRITE) == 0) return;
-#else
-  (void)hi;
-#endif
-  for (uintptr_t a = lo < (uintptr_t)p ? (uintptr_t)p : lo; a < (uintptr_t)p + bytes; a = (a & ~(page - 1)) + page)
-    __atomic_fetch_or((unsigned char *)a, 0, __ATOMIC_RELAXED);
+  madvise((void *)lo, hi - lo, 23 /* MADV_POPULATE_WRITE, Linux 5.14 */); /* refused: only slower */
 }
 
 cudaError_t ensure_pinned(mcfl_ctx *c, size_t jobs, size_t outs) {
@@ -258,12 +252,6 @@ void add_walk_limits(McflLaunch &L, const mcfl_medium *m) {
 void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool emission, unsigned long long *fhd,
                  bool exact = false) {
   L.uniform_medium = 1;
-  if (c->l2_window && c->l2_max_window) {
-    const size_t bytes = std::min<size_t>(m->labels.bytes, c->l2_max_window);
-    L.l2_base = m->labels.p;
-    L.l2_bytes = bytes;
-    L.l2_hit_ratio = (float)std::min(1.0, (double)c->l2_persist_bytes / (double)bytes);
-  }
   McflMedium &u = L.med;
   u.labels = m->labels.as<uint8_t>();
   u.prop = m->prop_of(emission, exact);
@@ -278,6 +266,13 @@ void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool em
     u.tile_bytes = (uint32_t)m->tiles.bytes;
   } else {
     L.plain = 0; /* no tiles (ensure_tiles was not called): the transport kernel */
+  }
+  if (c->l2_window && c->l2_max_window) { /* over the array that every pass reads */
+    const mcfl::DevBuf &read = L.plain && !exact ? m->tiles : m->labels;
+    const size_t bytes = std::min<size_t>(read.bytes, c->l2_max_window);
+    L.l2_base = read.p;
+    L.l2_bytes = bytes;
+    L.l2_hit_ratio = (float)std::min(1.0, (double)c->l2_persist_bytes / (double)bytes);
   }
   L.w_event = m->w_event[emission];
   u.fhd = fhd;
