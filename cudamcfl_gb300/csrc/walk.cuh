@@ -686,6 +686,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
       uint32_t vi, g;
       Rec c;
       real u_hg, cosp, sinp;
+      /* Whether a pass is special.  A direction can become NaN (a cosine that
+       * rounds beyond 1), and its photon walks on, outside the grid, until
+       * the roulette: about one photon in 1e5, for some 1e4 passes, so these
+       * passes have to be common where they can.  A NaN position is no reason
+       * (fminf passes it over); a NaN direction is one in fast math, where the
+       * deflection then starts as from the z axis and gives a number again. */
+      auto needs_decisions = [&]() {
+        return !(fminf(zn, s) > MCFL_C(0.0)) || (MCFL_EXACT_MATH ? q <= MCFL_C(0.0) : !(q > MCFL_C(0.0))) ||
+               zn >= m.esp || p.weight <= w_event || left == 0u;
+      };
       /* the hitting density at a point that is not a common pass's end */
       auto tally_at = [&](real x, real y, real z, uint32_t w) {
         if ((kPhd || (!kNoPhd && m.fhd)) && MCFL_FABS(x) < m.hx && MCFL_FABS(y) < m.hy && z < m.esp)
@@ -711,7 +721,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
          * hint) */
         asm("ld.global.nc.L1::evict_last.u8 %0, [%1];" : "=r"(g) : "l"(at));
         q = fp_one_minus_sq(p.dz);
-        special = !(fminf(fminf(zn, s), q) > MCFL_C(0.0)) || !(zn < m.esp) || p.weight <= w_event || left == 0u;
+        special = needs_decisions();
         if (__any_sync(live, special)) break;
         --left;
         walk_draw(r, u_hg, cosp, sinp);
@@ -732,7 +742,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
        * reference's sequence up to the deflection, which all lanes then make
        * together ---- */
       inside = inside && zn < m.esp;
-      special = !(fminf(fminf(zn, s), q) > MCFL_C(0.0)) || !(zn < m.esp) || p.weight <= w_event || left == 0u;
+      special = needs_decisions();
       bool spin_now = true;
       const uint32_t lab = inside ? g : 1u;
       if (special) {
