@@ -152,6 +152,14 @@ typedef struct McflMedium {
 
 #define MCFL_FREE_MAX 31
 
+/* How the walk kernel tallies the hitting density: one add per pass
+ * (kWalkAdds); none (kWalkNone: no job tallies it); or the weights of a lane's
+ * successive passes in one voxel summed in registers and added when the voxel
+ * changes (kWalkRuns): under a beam the adds of all photons go to a few voxels
+ * and queue up in L2.  The same integer sums.  lit_columns (run.cpp) has the
+ * rule and both sides. */
+enum { kWalkAdds = 0, kWalkNone = 1, kWalkRuns = 2 };
+
 typedef struct McflLaunch {
   const McflJob *jobs;   /* job slots */
   const uint32_t *order; /* slots sorted by ticket_begin, or NULL: slots 0..n_jobs-1 in order */
@@ -187,8 +195,9 @@ typedef struct McflLaunch {
   uint32_t relaunch_min;
   /* plain: every medium of the launch is plain (mcfl_medium::plain), so the
    * walk kernel runs it; w_event: the weight up to which it takes the event
-   * code; sm_count: the GPU's SMs */
-  uint32_t plain, w_event, sm_count;
+   * code; sm_count: the GPU's SMs; phd_runs: the hitting density is summed
+   * over a photon's passes in one voxel before it is added */
+  uint32_t plain, w_event, sm_count, phd_runs;
   float l2_hit_ratio;      /* host side: persisting-L2 window over [l2_base, +l2_bytes) when l2_bytes > 0 */
   const void *l2_base;
   unsigned long long l2_bytes;

@@ -18,6 +18,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <functional>
 #include <string>
@@ -247,6 +248,23 @@ void add_walk_limits(McflLaunch &L, const mcfl_medium *m) {
   L.w_event = std::max(L.w_event, m->w_event[0]);
 }
 
+/* Voxel columns under the source, about: of a collimated beam (its radius is
+ * 0.03 cm sqrt(-ln u)) the square of 0.1 cm that holds nine photons of ten.
+ * Up to kRunColumns of them the hitting density is summed over a photon's
+ * passes in one voxel (kWalkRuns in walk.cuh): then the adds of the photons
+ * under the source to the same few voxels set the launch's time.  GB300, 3e6
+ * photons in a slab of 4 x 4 x 2 cm, an add per pass and summed: beams on 24,
+ * 64, 128, 200 and 256 voxels a side 92.3 > 20.3, 20.1 > 15.4, 16.8 > 15.9,
+ * 16.5 > 16.1, 16.4 > 16.2 ms (variant 1: 17.7 > 16.0 at 200); wide field over
+ * the whole face, 625 columns 41.0 > 15.0 ms, but 2401 columns 14.6 < 14.8 and
+ * 40401 columns 15.6 < 15.9. */
+constexpr double kRunColumns = 1024.0;
+double lit_columns(const mcfl_medium *m, const mcfl_run_desc &run) {
+  const bool wide = run.source.kind == MCFL_SOURCE_WIDEFIELD;
+  const double w = wide ? std::fabs((double)run.source.width) : 0.1, h = wide ? std::fabs((double)run.source.height) : 0.1;
+  return (w * m->gx + 1.0) * (h * m->gy + 1.0);
+}
+
 /* Every job of the launch uses medium m with one photon-hitting-density
  * tally (or none): the medium travels in the kernel parameters. */
 void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool emission, unsigned long long *fhd,
@@ -423,6 +441,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
   const int grid_exc = c->grid_for(true, &block_exc, nullptr, timed, exact);
   const unsigned long long photons = run->photons;
   const unsigned per_voxel = run->photons_per_voxel;
+  const uint32_t phd_runs = fluence && lit_columns(m, *run) <= kRunColumns ? 1u : 0u;
   auto record = [&](cudaStream_t st, unsigned *k) -> cudaError_t {
     cudaError_t e;
 #define REC(x)                   \
@@ -445,6 +464,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
     L.ticket_counter = cnt + 0;
     L.ticket_end = photons;
     set_uniform(c, L, m, false, fluence ? c->fhd.as<unsigned long long>() : nullptr, exact);
+    L.phd_runs = phd_runs;
     L.time_on = timed ? 1u : 0u;
     L.exact_step = exact ? 1u : 0u;
     REC(record_event(c->ev[0], st));
@@ -483,7 +503,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
                                    (unsigned long long)c->variant_code(true),
                                    (unsigned long long)c->l2_window, tsize, (unsigned long long)grid_exc,
                                    (unsigned long long)block_exc, (unsigned long long)exact, m->serial,
-                                   c->relaunch});
+                                   c->relaunch, phd_runs});
   rc = replay(c, &c->graph_run, &c->graph_run_key, &c->graph_run_kernels, key, record);
   if (rc != MCFL_OK) return rc;
 

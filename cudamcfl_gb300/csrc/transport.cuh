@@ -1638,28 +1638,38 @@ static int mixed_variant_code(uint32_t v) {
 #if MCFL_F64
 /* the double-precision build runs the transport kernel's own pass throughout */
 static bool is_walk(int, bool) { return false; }
-static TransportKernel walk_of(int, bool) { return nullptr; }
+static TransportKernel walk_of(int, int) { return nullptr; }
 #else
 static bool is_walk(int variant, bool plain) { return plain && variant >= -4 && variant <= 3; }
 
-static TransportKernel walk_of(int variant, bool no_phd) {
+template <int kThreads, int kMinBlocks>
+static TransportKernel walk_shape(int tally) {
+  return tally == kWalkNone   ? MCFL_WALK_NAME<true, false, kWalkNone, kThreads, kMinBlocks>
+         : tally == kWalkRuns ? MCFL_WALK_NAME<true, false, kWalkRuns, kThreads, kMinBlocks>
+                              : MCFL_WALK_NAME<true, false, kWalkAdds, kThreads, kMinBlocks>;
+}
+
+static TransportKernel walk_of(int variant, int tally) {
   switch (variant) {
-  case -2: return MCFL_WALK_NAME<false, true, false, 256, 2>;
-  case -1: return MCFL_WALK_NAME<false, false, false, 256, 3>;
-  case -3: return MCFL_WALK_NAME<false, false, false, 256, 4>;
-  case -4: return MCFL_WALK_NAME<false, false, false, 128, 7>;
-  case 0: return no_phd ? MCFL_WALK_NAME<true, false, true, 256, 4> : MCFL_WALK_NAME<true, false, false, 256, 4>;
-  case 1: return no_phd ? MCFL_WALK_NAME<true, false, true, 256, 5> : MCFL_WALK_NAME<true, false, false, 256, 5>;
-  case 2: return no_phd ? MCFL_WALK_NAME<true, false, true, 128, 9> : MCFL_WALK_NAME<true, false, false, 128, 9>;
-  case 3: return MCFL_WALK_NAME<true, true, false, 256, 3>;
+  case -2: return MCFL_WALK_NAME<false, true, kWalkAdds, 256, 2>;
+  case -1: return MCFL_WALK_NAME<false, false, kWalkAdds, 256, 3>;
+  case -3: return MCFL_WALK_NAME<false, false, kWalkAdds, 256, 4>;
+  case -4: return MCFL_WALK_NAME<false, false, kWalkAdds, 128, 7>;
+  case 0: return walk_shape<256, 4>(tally);
+  case 1: return walk_shape<256, 5>(tally);
+  case 2: return walk_shape<128, 9>(tally);
+  case 3:
+    return tally == kWalkRuns ? MCFL_WALK_NAME<true, true, kWalkRuns, 256, 3>
+                              : MCFL_WALK_NAME<true, true, kWalkAdds, 256, 3>;
   default: return nullptr;
   }
 }
 #endif
 
-static TransportKernel kernel_of(int variant, int *threads, bool plain = false, bool no_phd = false) {
+static TransportKernel kernel_of(int variant, int *threads, bool plain = false, bool no_phd = false,
+                                 bool runs = false) {
   *threads = variant == -4 || variant == 2 ? 128 : 256;
-  if (is_walk(variant, plain)) return walk_of(variant, no_phd);
+  if (is_walk(variant, plain)) return walk_of(variant, no_phd ? kWalkNone : runs ? kWalkRuns : kWalkAdds);
   switch (variant) {
   case -2: return MCFL_KERNEL_NAME<false, true, 0, 256, 2>;
   case -1: return MCFL_KERNEL_NAME<false, false, 0, 256, 3>;
@@ -1735,7 +1745,7 @@ extern "C" cudaError_t MCFL_LAUNCHER(const McflLaunch *L, int grid, int block, c
   /* variants 0..2 without a hitting-density tally run their instantiations
    * that compile none */
   const bool no_phd = v >= 0 && v <= 2 && !L->med.fhd;
-  const TransportKernel fn = kernel_of(v, &t, L->plain != 0, no_phd);
+  const TransportKernel fn = kernel_of(v, &t, L->plain != 0, no_phd, L->phd_runs != 0);
   if (!fn || block > t) return cudaErrorInvalidValue;
   const bool walk = is_walk(v, L->plain != 0);
   cudaLaunchConfig_t cfg;

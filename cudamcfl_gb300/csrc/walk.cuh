@@ -227,10 +227,11 @@ static size_t walk_dynamic(bool uniform, bool time, int block, uint32_t n_labels
 
 /* kUniform: the medium comes from the launch parameters and the label records
  * from shared memory; otherwise (mixed media) both come from the photon's
- * job.  kTime: carries the time of flight.  kNoPhd: no job tallies the
- * hitting density. */
-template <bool kUniform, bool kTime, bool kNoPhd, int kThreads, int kMinBlocks>
+ * job.  kTime: carries the time of flight.  kTally: how the hitting density
+ * is tallied. */
+template <bool kUniform, bool kTime, int kTally, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunch L) {
+  constexpr bool kNoPhd = kTally == kWalkNone, kRuns = kTally == kWalkRuns;
   constexpr bool kDirs = kNoPhd && !kTime; /* only these launches have emitting voxels */
   constexpr bool kPhd = kUniform && !kTime && !kNoPhd; /* such a launch always tallies it */
   /* After a pass with decisions in which no photon ended, back to the common
@@ -333,6 +334,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
   real nl = MCFL_C(1.0);     /* -log of the pass's step draw */
   real mutr = MCFL_C(0.0);   /* 1/mu_t of the photon's label */
   uint32_t pst = 0;          /* the photon's passes */
+  uint32_t run_at = 0;       /* kWalkRuns: the voxel and the weight summed there */
+  unsigned long long run_w = 0ull;
   uint32_t pst0 = 0;         /* slices: passes before this one */
   uint64_t k = 0;
   auto job_of = [&]() -> const McflJob * { return &L.jobs[job]; };
@@ -731,7 +734,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
         p.y = yn;
         p.z = zn;
         if constexpr (kTime) p.tof += tof_fs(fp_mul(s, c.b.w)); /* every label has this index */
-        if ((kPhd || (!kNoPhd && m.fhd)) && inside) atomicAdd(&m.fhd[vi], (unsigned long long)p.weight);
+        if constexpr (kRuns) {
+          const uint32_t w = inside ? p.weight : 0u;
+          const bool same = vi == run_at || !inside;
+          if (!same) atomicAdd(&m.fhd[run_at], run_w);
+          run_w = (same ? run_w : 0ull) + w;
+          run_at = same ? run_at : vi;
+        } else if ((kPhd || (!kNoPhd && m.fhd)) && inside) {
+          atomicAdd(&m.fhd[vi], (unsigned long long)p.weight);
+        }
         p.weight -= MCFL_R2U_RU(fp_mul(c.a.y, MCFL_U2R_RN(p.weight)));
         walk_spin<false, kSplit>(p, c, u_hg, cosp, sinp, q);
         mutr = c.a.x;
@@ -868,6 +879,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
     if (sliced) w.it = it + made;
     __syncwarp();
   }
+  if (kRuns && run_w) atomicAdd(&m.fhd[run_at], run_w);
   if (alive) {
     steps += pst - pst0; /* passes of the photon parked by this slice */
     absorbed -= p.weight;

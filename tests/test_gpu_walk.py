@@ -173,3 +173,25 @@ def test_last_photons_gathered_bit_identical_to_oracle(name, gpu_ctx, oracle, ta
     res = gpu_ctx.run(med, case.run_desc(31, 32))
     med.free()
     _compare(res, ref, emission=name != "layered")
+
+
+# hitting densities summed over a photon's passes in a voxel (few voxel columns under the source) and added pass by pass
+@pytest.mark.gpu
+@pytest.mark.parametrize("timed", [False, True])
+@pytest.mark.parametrize("width", [0.0, 0.5, 2.0, 3.9])
+def test_hitting_density_equals_branching_pass(width, timed, gpu_ctx):
+    lab, bulks, geo = _plain(40, 40, 8)
+    med = gpu_ctx.medium(lab, bulks, **geo)
+    tdet = (0.1, -0.05, 2, 2, 0.25, 0.25, 0.15, 0, 20, 150000) if timed else None
+    rd = mc.run_desc(20011, det=mc.Detector(0.0, 0.0, 0.05, 0.05, 30, 30), fluence=1, seed_exc=5, tdet=tdet,
+                     kind=mc.SOURCE_WIDEFIELD if width else mc.SOURCE_GAUSS_BEAM, width=width, height=width)
+    got = []
+    try:
+        for form in (0, 1):
+            gpu_ctx.set_option("pass_form", form)
+            got.append(gpu_ctx.run(med, rd))
+    finally:
+        gpu_ctx.set_option("pass_form", 0)
+        med.free()
+    assert np.array_equal(got[0].fhd, got[1].fhd) and got[0].fhd.any()
+    assert np.array_equal(got[0].Rd, got[1].Rd) and got[0].stats_exc == got[1].stats_exc
