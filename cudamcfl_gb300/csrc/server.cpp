@@ -16,8 +16,14 @@
  *      their memory and slot are released.
  * New work therefore joins the running batch at the next slice (every few
  * milliseconds) while earlier requests are still in flight, and a request's
- * photons draw the same random streams whatever else shares the GPU, so its
- * tallies equal those of running it alone bit for bit.
+ * photons draw the same random streams whatever else shares the GPU, so in
+ * strict math its tallies equal those of running it alone bit for bit.  In
+ * fast math they do so for plain media, whose pass the walk kernel, the
+ * transport kernel and their mixed-media forms round alike (a slice runs the
+ * walk kernel when every medium in flight is plain; a photon may be parked by
+ * one kernel and resumed by the other); on other media the mixed-media
+ * kernel may contract an expression in another way than the single-medium
+ * one, and the two agree statistically.
  */
 #include <cuda_runtime.h>
 

@@ -415,7 +415,12 @@ int mcfl_batch_run(mcfl_ctx *ctx, const mcfl_medium *medium, const mcfl_run_desc
 /* mcfl_batch_run with a medium per simulation (media[i] for runs[i]): many
  * sources, media and budgets in one persistent launch, replayed as a CUDA
  * graph; jobs on different media run the mixed-media kernel variant (each job
- * carries its medium).  Layered media batch only with their own medium. */
+ * carries its medium).  Layered media batch only with their own medium.  In
+ * strict math each simulation's images equal those of its run alone bit for
+ * bit; in fast math they do so for media whose labels all scatter, none of
+ * them isotropically, and share one refractive index, and on others agree
+ * statistically (the two kernels' roundings may differ).  The same holds for
+ * the server's results below. */
 int mcfl_batch_run_media(mcfl_ctx *ctx, const mcfl_medium *const *media, const mcfl_run_desc *runs, int n,
                          int schedule, mcfl_run_out *outs, float *gpu_ms);
 
