@@ -225,6 +225,7 @@ extern "C" long long mcfl_get_option(mcfl_ctx *c, const char *key) {
   if (k == "mixed_variant") return c->mixed_variant;
   if (k == "step_cap") return c->step_cap;
   if (k == "l2_window") return c->l2_window;
+  if (k == "l2_window_bytes") return (long long)c->window_bytes;
   if (k == "relaunch") return c->relaunch;
   if (k == "graphs") return c->use_graphs;
   if (k == "graph_failed") return c->graph_error.empty() ? 0 : 1;
@@ -460,5 +461,7 @@ extern "C" void mcfl_medium_free(mcfl_medium *m) {
   delete m;
 }
 
-extern "C" size_t mcfl_medium_bytes(const mcfl_medium *m) { return m ? m->bytes : 0; }
+extern "C" size_t mcfl_medium_bytes(const mcfl_medium *m) {
+  return m ? m->bytes + m->tiles.bytes + m->lab16.bytes : 0;
+}
 

@@ -102,8 +102,8 @@ int run_single_voxel_emission(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_
  * the medium's first such run (synchronously on the context's stream) */
 int ensure_free_map(mcfl_ctx *c, const mcfl_medium *m);
 
-/* run.cpp: the label tiles of the walk kernel, built on a plain medium's
- * first single-medium run (in the order of the context's stream) */
+/* run.cpp: the label tiles of the walk kernel (in the order of the context's
+ * stream); without room for them none are built and MCFL_OK is returned */
 int ensure_tiles(mcfl_ctx *c, const mcfl_medium *m);
 
 /* mci.cpp */
@@ -204,6 +204,7 @@ struct mcfl_ctx {
   int l2_window = 0;            /* 1: persisting-L2 window over the medium's labels */
   size_t l2_persist_bytes = 0;  /* persisting set-aside this context asked for */
   size_t l2_max_window = 0;     /* cudaDevAttrMaxAccessPolicyWindowSize */
+  size_t window_bytes = 0;      /* of the last single-medium launch set up (0: it had no window) */
   unsigned long long launches = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 

@@ -265,10 +265,46 @@ double lit_columns(const mcfl_medium *m, const mcfl_run_desc &run) {
   return (w * m->gx + 1.0) * (h * m->gy + 1.0);
 }
 
+/* Whether single-medium launches over m run the walk kernel.  Decided here,
+ * once: the label tiles, the L2 window and the launcher follow it.  The other
+ * pass and tally forms, voxel-boundary stepping and FP64 run the transport
+ * kernel; a timed launch has one form only. */
+bool walks(const mcfl_ctx *c, const mcfl_medium *m, bool emission, bool timed, bool stepping) {
+  return m->plain[emission] && !stepping && c->math != MCFL_MATH_F64 && (timed || c->variant_code() < MCFL_N_VARIANTS);
+}
+
+/* Reserves the buffers of a run over the given media.  Label tiles are a
+ * convenience: where the device has no room left, they are given back first,
+ * and the run takes the transport kernel unless they fit beside the buffers
+ * after all. */
+typedef std::vector<std::pair<mcfl::DevBuf *, size_t>> Buffers;
+int reserve_for(const mcfl_ctx *c, const mcfl_medium *const *media, int n, const Buffers &want) {
+  auto reserve = [&]() -> cudaError_t {
+    for (const auto &b : want) {
+      const cudaError_t e = b.first->reserve(b.second);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  };
+  cudaError_t e = reserve();
+  bool released = false;
+  for (int i = 0; e == cudaErrorMemoryAllocation && i < n; ++i)
+    if (media[i]->tiles.p) {
+      if (!released) cudaStreamSynchronize(c->stream);
+      released = true;
+      media[i]->tiles.release();
+    }
+  if (released) {
+    cudaGetLastError();
+    e = reserve();
+  }
+  return e == cudaSuccess ? MCFL_OK : cuda_fail(e, "run buffers");
+}
+
 /* Every job of the launch uses medium m with one photon-hitting-density
  * tally (or none): the medium travels in the kernel parameters. */
-void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool emission, unsigned long long *fhd,
-                 bool exact = false) {
+void set_uniform(mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool emission, unsigned long long *fhd, bool timed,
+                 bool exact) {
   L.uniform_medium = 1;
   McflMedium &u = L.med;
   u.labels = m->labels.as<uint8_t>();
@@ -276,22 +312,24 @@ void set_uniform(const mcfl_ctx *c, McflLaunch &L, const mcfl_medium *m, bool em
   u.lab = m->lab_of(emission, exact);
   u.lab16 = exact ? m->lab16.as<uint16_t>() : nullptr;
   u.n_labels = (uint32_t)m->n_bulks + 2u;
-  L.plain = m->plain[emission] ? 1u : 0u;
-  if (m->tiles.p) {
+  /* without tiles (no room for them) the transport kernel runs the medium */
+  L.plain = m->tiles.p && walks(c, m, emission, timed, exact) ? 1u : 0u;
+  if (L.plain) {
     u.tiles = m->tiles.as<uint8_t>();
     u.tile_y = 16u * (uint32_t)(m->nx + 1) - 16u;
     u.tile_z = 16u * (uint32_t)(m->nx + 1) * (uint32_t)(m->ny / 4 + 1) - 4u;
     u.tile_bytes = (uint32_t)m->tiles.bytes;
-  } else {
-    L.plain = 0; /* no tiles (ensure_tiles was not called): the transport kernel */
   }
-  if (c->l2_window && c->l2_max_window) { /* over the array that every pass reads */
-    const mcfl::DevBuf &read = L.plain && !exact ? m->tiles : m->labels;
+  L.l2_base = nullptr;
+  L.l2_bytes = 0;
+  if (c->l2_window && c->l2_max_window) { /* over the label array that the launch's kernel reads */
+    const mcfl::DevBuf &read = L.plain ? m->tiles : m->labels;
     const size_t bytes = std::min<size_t>(read.bytes, c->l2_max_window);
     L.l2_base = read.p;
     L.l2_bytes = bytes;
     L.l2_hit_ratio = (float)std::min(1.0, (double)c->l2_persist_bytes / (double)bytes);
   }
+  c->window_bytes = (size_t)L.l2_bytes;
   L.w_event = m->w_event[emission];
   u.fhd = fhd;
   u.hx = m->hx;
@@ -320,8 +358,8 @@ int mcfl::ensure_free_map(mcfl_ctx *c, const mcfl_medium *m) {
   if (m->lab16.p) return MCFL_OK;
   const size_t n = (size_t)m->total;
   mcfl::DevBuf tmp;
-  MCFL_CUDA_TRY(tmp.reserve(2 * n));
-  MCFL_CUDA_TRY(m->lab16.reserve(2 * n));
+  const int rc = reserve_for(c, &m, 1, {{&tmp, 2 * n}, {&m->lab16, 2 * n}});
+  if (rc != MCFL_OK) return rc;
   cudaError_t e = mcfl_launch_free_map(m->labels.as<uint8_t>(), m->nx, m->ny, m->nz, tmp.as<uint8_t>(),
                                        m->lab16.as<uint16_t>(), c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -332,12 +370,18 @@ int mcfl::ensure_free_map(mcfl_ctx *c, const mcfl_medium *m) {
   return MCFL_OK;
 }
 
-/* The walk kernel's label tiles, built on a plain medium's first
- * single-medium run (before any recorded graph uses them). */
+/* The walk kernel's label tiles, built before the medium's first launch of
+ * that kernel (and before a recorded graph uses them), after the run's own
+ * buffers: where the device has no room for them the run goes on without. */
 int mcfl::ensure_tiles(mcfl_ctx *c, const mcfl_medium *m) {
-  if (m->tiles.p || !(m->plain[0] || m->plain[1])) return MCFL_OK;
+  if (m->tiles.p) return MCFL_OK;
   const size_t n = (size_t)tile_bytes_of(m->nx, m->ny, m->nz);
-  MCFL_CUDA_TRY(m->tiles.reserve(n));
+  const cudaError_t room = m->tiles.reserve(n);
+  if (room == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return MCFL_OK;
+  }
+  MCFL_CUDA_TRY(room);
   const cudaError_t e = mcfl_launch_tiles(m->labels.as<uint8_t>(), m->nx, m->ny, m->nz, m->total,
                                           m->tiles.as<uint8_t>(), (uint32_t)n, c->stream);
   if (e != cudaSuccess) {
@@ -360,31 +404,33 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   cudaGetLastError();
   if (run->exact_stepping && (rc = ensure_free_map(c, m)) != MCFL_OK) return rc;
-  if (!run->exact_stepping && (rc = ensure_tiles(c, m)) != MCFL_OK) return rc;
   cudaStream_t s = c->stream;
   const size_t xy = (size_t)det.nx + (size_t)det.nx * det.ny;
   const size_t nv = m->total;
-
-  MCFL_CUDA_TRY(c->R.reserve(xy * 8));
-  MCFL_CUDA_TRY(c->T.reserve(xy * 8));
-  MCFL_CUDA_TRY(c->stats.reserve(2 * MCFL_ST_COUNT * 8));
-  MCFL_CUDA_TRY(c->jobs.reserve(2 * sizeof(McflJob)));
-  if (fluence) MCFL_CUDA_TRY(c->fhd.reserve(nv * 8));
-  if (emission) {
-    MCFL_CUDA_TRY(c->R128.reserve(xy * 16));
-    MCFL_CUDA_TRY(c->T128.reserve(xy * 16));
-    MCFL_CUDA_TRY(c->vox.reserve(nv * 4));
-    MCFL_CUDA_TRY(c->q.reserve(nv * 8));
-    MCFL_CUDA_TRY(c->block_counts.reserve(emission_prep_blocks((uint32_t)nv) * 4 + 16));
-  }
-  const size_t nout = 2 * MCFL_ST_COUNT + 4;
-  MCFL_CUDA_TRY(ensure_pinned(c, 2, nout));
   const mcfl_time_detectors &td = run->tdet;
   const bool timed = td.nx > 0;
   const size_t tsize = timed ? (size_t)td.nx * td.ny * td.bins : 0;
+  const size_t nd = !out ? 0
+                         : (out->R ? xy : 0) + (out->T ? xy : 0) + (out->phd && fluence ? nv : 0) +
+                               (emission ? (out->flR ? xy : 0) + (out->flT ? xy : 0) : 0);
+  Buffers want = {
+      {&c->R, xy * 8}, {&c->T, xy * 8}, {&c->stats, 2 * MCFL_ST_COUNT * 8}, {&c->jobs, 2 * sizeof(McflJob)}};
+  if (fluence) want.push_back({&c->fhd, nv * 8});
+  if (emission)
+    want.insert(want.end(), {{&c->R128, xy * 16},
+                             {&c->T128, xy * 16},
+                             {&c->vox, nv * 4},
+                             {&c->q, nv * 8},
+                             {&c->block_counts, emission_prep_blocks((uint32_t)nv) * 4 + 16}});
+  if (timed) want.insert(want.end(), {{&c->tpos, (size_t)(td.nx + td.ny) * 4}, {&c->tarr, tsize * 8}});
+  if (nd) want.push_back({&c->outd, nd * 8});
+  if ((rc = reserve_for(c, &m, 1, want)) != MCFL_OK) return rc;
+  const size_t nout = 2 * MCFL_ST_COUNT + 4;
+  MCFL_CUDA_TRY(ensure_pinned(c, 2, nout));
+  if ((walks(c, m, false, timed, run->exact_stepping) || (emission && walks(c, m, true, false, run->exact_stepping))) &&
+      (rc = ensure_tiles(c, m)) != MCFL_OK)
+    return rc;
   if (timed) {
-    MCFL_CUDA_TRY(c->tpos.reserve((size_t)(td.nx + td.ny) * 4));
-    MCFL_CUDA_TRY(c->tarr.reserve(tsize * 8));
     std::vector<float> pos((size_t)(td.nx + td.ny));
     time_positions(td, pos.data(), pos.data() + td.nx);
     MCFL_CUDA_TRY(cudaMemcpyAsync(c->tpos.p, pos.data(), pos.size() * 4, cudaMemcpyHostToDevice, s));
@@ -463,7 +509,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
     L.n_jobs = 1;
     L.ticket_counter = cnt + 0;
     L.ticket_end = photons;
-    set_uniform(c, L, m, false, fluence ? c->fhd.as<unsigned long long>() : nullptr, exact);
+    set_uniform(c, L, m, false, fluence ? c->fhd.as<unsigned long long>() : nullptr, timed, exact);
     L.phd_runs = phd_runs;
     L.time_on = timed ? 1u : 0u;
     L.exact_step = exact ? 1u : 0u;
@@ -482,7 +528,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
       Lf.jobs = c->jobs.as<McflJob>() + 1;
       Lf.ticket_counter = cnt + 1;
       Lf.ticket_end_dev = cnt + 3;
-      set_uniform(c, Lf, m, true, nullptr, exact);
+      set_uniform(c, Lf, m, true, nullptr, false, exact);
       Lf.variant = (uint32_t)c->variant_code(true);
       REC(record_event(c->ev[2], st));
       REC(launch_fn(c->math)(&Lf, grid, block, st));
@@ -496,7 +542,7 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
   };
   const std::string key = ptr_key({m, c->R.p, c->T.p, c->fhd.p, c->R128.p, c->T128.p, c->vox.p, c->q.p, c->jobs.p,
                                    c->h_jobs, c->h_out, c->stats.p, c->block_counts.p, (const void *)s,
-                                   timed ? c->tarr.p : nullptr},
+                                   timed ? c->tarr.p : nullptr, m->tiles.p},
                                   {xy, nv, (unsigned long long)emission, (unsigned long long)fluence, photons,
                                    per_voxel, (unsigned long long)c->math, (unsigned long long)grid,
                                    (unsigned long long)block, c->step_cap, (unsigned long long)c->variant_code(),
@@ -525,9 +571,6 @@ extern "C" int mcfl_run(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *
       touch_pages(out->flT128, xy * 16);
     }
     if (timed) touch_pages(out->time_xyt, tsize * 8);
-    size_t nd = (out->R ? xy : 0) + (out->T ? xy : 0) + (out->phd && fluence ? nv : 0) +
-                (emission ? (out->flR ? xy : 0) + (out->flT ? xy : 0) : 0);
-    if (nd) MCFL_CUDA_TRY(c->outd.reserve(nd * 8));
     double *dd = c->outd.as<double>();
     size_t off = 0;
     const double scale2 = ((double)0xFFFFFFFF * (double)photons) * (double)det.dx * (double)det.dy;
@@ -623,20 +666,9 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
   }
   MCFL_CUDA_TRY(cudaSetDevice(c->device));
   cudaGetLastError();
-  if (!exact)
-    for (int i = 0; i < n; ++i) {
-      const int rct = uniform || schedule == MCFL_SCHEDULE_PLAIN ? ensure_tiles(c, media[i]) : MCFL_OK;
-      if (rct != MCFL_OK) return rct;
-    }
   cudaStream_t s = c->stream;
   const size_t xy = (size_t)det.nx + (size_t)det.nx * det.ny;
   const size_t N = (size_t)n;
-  MCFL_CUDA_TRY(c->bR.reserve(N * xy * 8));
-  MCFL_CUDA_TRY(c->bT.reserve(N * xy * 8));
-  MCFL_CUDA_TRY(c->bstats.reserve(N * MCFL_ST_COUNT * 8));
-  MCFL_CUDA_TRY(c->bcnt.reserve(N * 8 + 8));
-  MCFL_CUDA_TRY(c->jobs.reserve(N * sizeof(McflJob) + sizeof(McflJob)));
-  MCFL_CUDA_TRY(ensure_pinned(c, N, N * MCFL_ST_COUNT + N + 8));
   /* time-resolved detectors: each timed run's histogram and disc positions
    * at its own offset in one buffer */
   std::vector<size_t> toff(N + 1, 0), poff(N + 1, 0);
@@ -647,9 +679,25 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
   }
   const size_t tsize = toff[N];
   const bool timed = tsize > 0;
+  bool any_norm = false;
+  for (int i = 0; outs && i < n; ++i) any_norm |= (outs[i].R || outs[i].T);
+  Buffers want = {{&c->bR, N * xy * 8},
+                  {&c->bT, N * xy * 8},
+                  {&c->bstats, N * MCFL_ST_COUNT * 8},
+                  {&c->bcnt, N * 8 + 8},
+                  {&c->jobs, (N + 1) * sizeof(McflJob)}};
+  if (timed) want.insert(want.end(), {{&c->tarr, tsize * 8}, {&c->tpos, poff[N] * 4}});
+  if (any_norm) want.insert(want.end(), {{&c->seg_scale, N * 8}, {&c->outd, 2 * N * xy * 8}});
+  if (const int rcw = reserve_for(c, media, n, want)) return rcw;
+  MCFL_CUDA_TRY(ensure_pinned(c, N, N * MCFL_ST_COUNT + N + 8));
+  if (uniform || schedule == MCFL_SCHEDULE_PLAIN)
+    for (int i = 0; i < n; ++i) {
+      /* the launch of a batch over one medium is timed as a whole */
+      const bool timed_i = schedule == MCFL_SCHEDULE_PLAIN ? runs[i].tdet.nx > 0 : timed;
+      const int rct = walks(c, media[i], false, timed_i, exact) ? ensure_tiles(c, media[i]) : MCFL_OK;
+      if (rct != MCFL_OK) return rct;
+    }
   if (timed) {
-    MCFL_CUDA_TRY(c->tarr.reserve(tsize * 8));
-    MCFL_CUDA_TRY(c->tpos.reserve(poff[N] * 4));
     std::vector<float> pos(poff[N]);
     for (int i = 0; i < n; ++i)
       if (runs[i].tdet.nx) time_positions(runs[i].tdet, pos.data() + poff[i], pos.data() + poff[i] + runs[i].tdet.nx);
@@ -708,7 +756,7 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
       L.n_jobs = (uint32_t)n;
       L.ticket_counter = c->bcnt.as<unsigned long long>();
       L.ticket_end = tickets;
-      if (uniform) set_uniform(c, L, m, false, nullptr, exact);
+      if (uniform) set_uniform(c, L, m, false, nullptr, timed, exact);
       else {
         L.variant = (uint32_t)c->mixed_code();
         L.plain = limits.plain;
@@ -725,7 +773,7 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
     };
     std::string key =
         ptr_key({m, c->bR.p, c->bT.p, c->bstats.p, c->bcnt.p, c->jobs.p, c->h_jobs, c->h_out, (const void *)s,
-                 timed ? c->tarr.p : nullptr},
+                 timed ? c->tarr.p : nullptr, m->tiles.p},
                 {N, xy, tickets, (unsigned long long)c->math, (unsigned long long)grid, (unsigned long long)block,
                  c->step_cap, (unsigned long long)c->variant_code(), (unsigned long long)c->l2_window,
                  (unsigned long long)uniform, (unsigned long long)exact, m->serial, tsize,
@@ -759,7 +807,7 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
       L.n_jobs = 1;
       L.ticket_counter = c->bcnt.as<unsigned long long>() + i;
       L.ticket_end = runs[i].photons;
-      set_uniform(c, L, media[i], false, nullptr, exact);
+      set_uniform(c, L, media[i], false, nullptr, timed_i, exact);
       L.exact_step = exact ? 1u : 0u;
       L.time_on = timed_i ? 1u : 0u;
       MCFL_CUDA_TRY(c->launch_transport(L, grid_one, block_one));
@@ -773,12 +821,8 @@ extern "C" int mcfl_batch_run_media(mcfl_ctx *c, const mcfl_medium *const *media
   if (gpu_ms) *gpu_ms = ms;
   bool capped = false;
   if (outs) {
-    bool any_norm = false;
-    for (int i = 0; i < n; ++i) any_norm |= (outs[i].R || outs[i].T);
     std::vector<double> scales(N);
     if (any_norm) {
-      MCFL_CUDA_TRY(c->seg_scale.reserve(N * 8));
-      MCFL_CUDA_TRY(c->outd.reserve(2 * N * xy * 8));
       for (int i = 0; i < n; ++i)
         scales[i] = ((double)0xFFFFFFFF * (double)runs[i].photons) * (double)runs[i].det.dx * (double)runs[i].det.dy;
       MCFL_CUDA_TRY(cudaMemcpyAsync(c->seg_scale.p, scales.data(), N * 8, cudaMemcpyHostToDevice, s));
@@ -839,11 +883,12 @@ extern "C" int mcfl_run_plain(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_
   exc.fluence = 1;
   rc = mcfl_run(c, m, &exc, nullptr);
   if (rc != MCFL_OK) return rc;
-  MCFL_CUDA_TRY(c->vox.reserve(nv * 4));
-  MCFL_CUDA_TRY(c->q.reserve(nv * 8));
-  MCFL_CUDA_TRY(c->block_counts.reserve(emission_prep_blocks((uint32_t)nv) * 4 + 16));
-  MCFL_CUDA_TRY(c->R128.reserve(xy * 16));
-  MCFL_CUDA_TRY(c->T128.reserve(xy * 16));
+  rc = reserve_for(c, &m, 1, {{&c->vox, nv * 4},
+                              {&c->q, nv * 8},
+                              {&c->block_counts, emission_prep_blocks((uint32_t)nv) * 4 + 16},
+                              {&c->R128, xy * 16},
+                              {&c->T128, xy * 16}});
+  if (rc != MCFL_OK) return rc;
   MCFL_CUDA_TRY(mcfl_launch_emission_prep(m->labels.as<uint8_t>(), m->fl.as<float2>(), c->fhd.as<unsigned long long>(),
                                           m->has_fmap ? m->fmap.as<float>() : nullptr, m->total, run->photons,
                                           run->photons_per_voxel, c->block_counts.as<uint32_t>(),
@@ -861,8 +906,9 @@ extern "C" int mcfl_run_plain(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_
   MCFL_CUDA_TRY(cudaMemsetAsync(c->T128.p, 0, xy * 16, s));
   MCFL_CUDA_TRY(cudaMemsetAsync(c->stats.as<unsigned long long>() + MCFL_ST_COUNT, 0, MCFL_ST_COUNT * 8, s));
   const size_t NL = (size_t)(nlist > 0 ? nlist : 0);
-  MCFL_CUDA_TRY(c->jobs.reserve((NL + 2) * sizeof(McflJob)));
-  MCFL_CUDA_TRY(c->bcnt.reserve(NL * 8 + 8));
+  rc = reserve_for(c, &m, 1, {{&c->jobs, (NL + 2) * sizeof(McflJob)}, {&c->bcnt, NL * 8 + 8}});
+  if (rc != MCFL_OK) return rc;
+  if (walks(c, m, true, false, run->exact_stepping) && (rc = ensure_tiles(c, m)) != MCFL_OK) return rc;
   MCFL_CUDA_TRY(ensure_pinned(c, NL + 2, 2 * MCFL_ST_COUNT + 8));
   McflJob t;
   std::memset(&t, 0, sizeof(t));
@@ -894,7 +940,7 @@ extern "C" int mcfl_run_plain(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_
     L.n_jobs = 1;
     L.ticket_counter = c->bcnt.as<unsigned long long>() + i;
     L.ticket_end = run->photons_per_voxel;
-    set_uniform(c, L, m, true, nullptr, run->exact_stepping != 0);
+    set_uniform(c, L, m, true, nullptr, false, run->exact_stepping != 0);
     L.exact_step = run->exact_stepping ? 1u : 0u;
     MCFL_CUDA_TRY(c->launch_transport(L, grid, block));
     MCFL_CUDA_TRY(cudaStreamSynchronize(s)); /* one simulation per call, as DoOneSimulationFl */
@@ -933,16 +979,18 @@ int mcfl::run_single_voxel_emission(mcfl_ctx *c, const mcfl_medium *m, const mcf
   if (run->exact_stepping) {
     const int rcm = ensure_free_map(c, m);
     if (rcm != MCFL_OK) return rcm;
-  } else {
+  }
+  const int rcw = reserve_for(c, &m, 1, {{&c->R128, xy * 16},
+                                         {&c->T128, xy * 16},
+                                         {&c->vox, 64},
+                                         {&c->q, 64},
+                                         {&c->stats, 2 * MCFL_ST_COUNT * 8},
+                                         {&c->jobs, 2 * sizeof(McflJob)}});
+  if (rcw != MCFL_OK) return rcw;
+  if (walks(c, m, false, false, run->exact_stepping)) {
     const int rct = ensure_tiles(c, m);
     if (rct != MCFL_OK) return rct;
   }
-  MCFL_CUDA_TRY(c->R128.reserve(xy * 16));
-  MCFL_CUDA_TRY(c->T128.reserve(xy * 16));
-  MCFL_CUDA_TRY(c->vox.reserve(64));
-  MCFL_CUDA_TRY(c->q.reserve(64));
-  MCFL_CUDA_TRY(c->stats.reserve(2 * MCFL_ST_COUNT * 8));
-  MCFL_CUDA_TRY(c->jobs.reserve(2 * sizeof(McflJob)));
   const uint64_t one = 1;
   MCFL_CUDA_TRY(cudaMemcpyAsync(c->vox.p, &voxel, 4, cudaMemcpyHostToDevice, s));
   MCFL_CUDA_TRY(cudaMemcpyAsync(c->q.p, &one, 8, cudaMemcpyHostToDevice, s));
@@ -970,7 +1018,7 @@ int mcfl::run_single_voxel_emission(mcfl_ctx *c, const mcfl_medium *m, const mcf
   L.n_jobs = 1;
   L.ticket_counter = c->counters.as<unsigned long long>();
   L.ticket_end = run->photons;
-  set_uniform(c, L, m, false, nullptr, run->exact_stepping != 0);
+  set_uniform(c, L, m, false, nullptr, false, run->exact_stepping != 0);
   L.exact_step = run->exact_stepping ? 1u : 0u;
   int block = 0;
   const int grid = c->grid_for(true, &block, nullptr, false, run->exact_stepping != 0);

@@ -375,6 +375,8 @@ int mcfl_medium_create_layered(mcfl_ctx *ctx, const mcfl_layered_desc *desc, mcf
  * come before mcfl_destroy of its context. */
 int mcfl_medium_create(mcfl_ctx *ctx, const mcfl_medium_desc *desc, mcfl_medium **medium);
 void mcfl_medium_free(mcfl_medium *medium);
+/* Device memory that the medium holds now: what mcfl_medium_create uploaded
+ * and, once a run has built them, the label tiles or the free-radius map. */
 size_t mcfl_medium_bytes(const mcfl_medium *medium);
 
 /* Builds the medium of a parsed .mci simulation (bulk method 2). */
