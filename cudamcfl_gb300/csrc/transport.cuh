@@ -735,11 +735,16 @@ __device__ __noinline__ void tally_time(const McflJob *J, real px, real py, uint
  * share their photons out evenly among as few warps as hold them (at least
  * kMeetWarps while there are photons for these), so that the long-lived
  * photons do not keep every warp issuing passes for one or two lanes.  The
- * photons move through kMeetPool entries of shared memory.  Measured in strict
- * math: 1e6 + 5e5 photons in a medium of several indices 24.4 + 21.6 -> 21.4 +
- * 19.2 ms; layered, 1e6 photons fast, 7.6 -> 7.15 ms.
- * Not in the fast build's voxelized kernels: the compiler contracts their
- * passes another way when code is added, and their results would change. */
+ * photons move through kMeetPool entries of shared memory.  Whole calls without
+ * and with it: strict math, several indices, 1e6 + 5e5 photons 43.8 -> 38.9 ms,
+ * a label free of scattering, 4e6 photons 28.8 -> 24.2, voxel-boundary stepping,
+ * 1e6 photons 36.5 -> 34.6; layered (one build, six media in turn) 1e6 photons
+ * fast 7.8 -> 7.4, strict 9.7 -> 9.2, 2000 photons 1.76 -> 1.63 ms.  The price is
+ * a test per pass: where photons live short (a slab of 0.5 cm, no hitting
+ * density, 256 x 4) 4e6 strict-math photons 11.1 -> 11.4 ms.
+ * Not in the fast build's voxelized kernels: their roundings are left to the
+ * compiler, which contracts the pass another way when code is added, so that
+ * results would change until each rounding is written out (as in walk.cuh). */
 __host__ __device__ constexpr bool meets(bool layered) { return !MCFL_F64 && (MCFL_EXACT_MATH || layered); }
 constexpr uint32_t kMeetPasses = 256u, kMeetWarps = 2u, kMeetPool = 64u;
 /* a run of few photons is spread over this many warps of each SM */
@@ -813,7 +818,7 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
   MovedStep *s_step = reinterpret_cast<MovedStep *>(s_moved + kMeetPool);
   __shared__ uint32_t s_live[kMeet ? kThreads / 32 : 1];
   __shared__ uint64_t s_tof[kMeet && kTime ? kMeetPool : 1];
-  bool tail = false, first = true;
+  bool first = true;
   uint32_t meet_in = 0;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned tib = threadIdx.x;
@@ -965,8 +970,7 @@ __global__ void __launch_bounds__(kThreads, MCFL_F64 ? 1 : kMinBlocks) MCFL_KERN
      * of any warp-wide operation inside the pass */
     unsigned live = kFull;
     const unsigned dead = __ballot_sync(kFull, !alive);
-    if (kMeet && (tail || (dead && ex0))) {
-      tail = true;
+    if (kMeet && ex0) { /* all tickets drawn: this warp's last draw left a lane free */
       if (meet_in == 0u || dead == kFull) {
         const unsigned n_warps = blockDim.x >> 5;
         const unsigned start = L.sm_count ? (blockIdx.x / L.sm_count) % n_warps : 0u;
