@@ -11,7 +11,8 @@
  *                   scheduled the reference's way (CUDAMCFLmain.cu:471-594):
  *                   one launch per emitting voxel.
  * Photon k of a simulation always uses stream (key, rng_offset + k), so the
- * schedules give bit-identical tallies; only their speed differs.
+ * schedules give bit-identical tallies and only their speed differs (fast math,
+ * several media in one launch: see mcfl_batch_run_media in mcfl.h).
  */
 #include <cuda_runtime.h>
 #include <sys/mman.h>
@@ -118,9 +119,16 @@ int check_run(const mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_desc *run)
   return MCFL_OK;
 }
 
-/* Brings the pages of an output buffer in while the GPU computes: a copy into
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23 /* Linux 5.14; older headers lack the name */
+#endif
+
+/* Brings the pages of an output buffer in while the GPU computes (mcfl_run and
+ * the batched schedule; the plain schedules copy as they are): a copy into
  * pages that the host has not written yet faults on the GPU side, about 50 us
  * for each page (26 ms for a fresh 32 MB array, 0.2 ms for a touched one).
+ * What a call gains depends on the state of the host's pages: on arrays whose
+ * pages are in place already, nothing.
  * The contents stay as they are.  Each page is faulted for writing at once; a
  * read before the write would map the zero page first and have its mapping
  * taken back from the GPU again (20 us for each page). */
@@ -129,7 +137,7 @@ void touch_pages(void *p, size_t bytes) {
   const long n = sysconf(_SC_PAGESIZE);
   const uintptr_t page = n > 0 ? (uintptr_t)n : 4096u;
   const uintptr_t lo = (uintptr_t)p & ~(page - 1), hi = ((uintptr_t)p + bytes + page - 1) & ~(page - 1);
-  madvise((void *)lo, hi - lo, 23 /* MADV_POPULATE_WRITE, Linux 5.14 */); /* refused: only slower */
+  madvise((void *)lo, hi - lo, MADV_POPULATE_WRITE); /* refused: only slower */
 }
 
 cudaError_t ensure_pinned(mcfl_ctx *c, size_t jobs, size_t outs) {
@@ -241,8 +249,8 @@ McflLaunch base_launch(mcfl_ctx *c) {
   return L;
 }
 
-/* A mixed-media launch takes up medium m: it is plain when all its media are,
- * its event weight the largest (L.plain starts as 1, L.w_event as 0). */
+/* A mixed-media launch takes up medium m: it is plain (and runs the walk
+ * kernel) when all its media are, its event weight the largest (L.plain starts as 1, L.w_event as 0). */
 void add_walk_limits(McflLaunch &L, const mcfl_medium *m) {
   if (!m->plain[0]) L.plain = 0;
   L.w_event = std::max(L.w_event, m->w_event[0]);

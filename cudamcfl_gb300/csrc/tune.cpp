@@ -4,14 +4,20 @@
  * The reference fixes its launch shape at compile time (128 blocks of 256
  * threads, CUDAMCFL.h:18-20).  The persistent kernel here is compiled in
  * several occupancy variants of the single-medium kernel (threads per block x
- * the blocks per SM the register budget is cut for), each with two forms of
- * the pass (arranged for the SIMT warp, or every test of the reference's
- * pass as its own branch) and two forms of the photon-hitting-density tally
- * (one atomic add per pass, or the sums of successive passes in one voxel
- * held in a register, a form of the branching pass), and can put a
- * persisting L2 access window on the labels and tallies; the SIMT-arranged
- * pass is also timed with the free lanes of a warp starting new photons in
- * pairs (option "relaunch" 2).  Which combination is fastest
+ * the blocks per SM the register budget is cut for), each in several forms,
+ * and can put a persisting L2 access window on the array of labels that the
+ * form reads.  The forms: the default pass (on plain media the walk kernel's,
+ * which sums the hitting density over a voxel or adds it pass by pass by the
+ * rule of lit_columns in run.cpp, no choice of the tuner's; on others the
+ * transport kernel's pass arranged for the SIMT warp); and, all in the
+ * transport kernel, every test of the reference's pass as its own branch
+ * ("pass_form" 1), and for runs that tally the hitting density the sums of
+ * successive passes in one voxel held in a register ("phd_agg" 1, a form of
+ * the branching pass) and the adds of a warp's lanes summed per voxel
+ * ("phd_agg" 2).  The default pass is also timed with the free lanes of a
+ * warp starting new photons in pairs (option "relaunch" 2).  On plain media
+ * the walk kernel was the faster one in every case measured (walk.cuh); the
+ * transport kernel's forms are timed all the same.  Which combination is fastest
  * depends on the medium (how often photons change label, how deep they go)
  * and on the emission/excitation mix, so the tuner times every combination on
  * a sample of the caller's own run and keeps the fastest in the context,
@@ -43,7 +49,7 @@ extern "C" int mcfl_autotune(mcfl_ctx *c, const mcfl_medium *m, const mcfl_run_d
   const int old_variant = c->variant, old_variant_fl = c->variant_fl, old_l2 = c->l2_window, old_agg = c->phd_agg,
             old_form = c->pass_form;
   const uint32_t old_relaunch = c->relaunch;
-  /* forms: 0 SIMT-arranged pass, 1 branching pass, and when the run tallies
+  /* forms: 0 the default pass, 1 branching pass, and when the run tallies
    * the hitting density 2 the branching pass with the register-held sums,
    * 3 the SIMT-arranged pass with the warp-aggregated adds; last, form 0
    * with relaunch 2.  Each with and without the L2 window. */

@@ -23,9 +23,9 @@
  *     alone and are computed while the end point's label is on its way.
  *   - Photons set up ahead.  A launch costs several hundred instructions
  *     (stream hashing, source sampling, label lookup) that one or two lanes
- *     of a warp used to run alone; here a warp sets up a queue of photons at
- *     once, all lanes working, in shared memory, and a free lane takes the
- *     next in a dozen loads.
+ *     of a warp used to run alone; here half of a warp's lanes set up a queue
+ *     of 16 photons at once in shared memory (32 gave no more), and a free
+ *     lane takes the next in a dozen loads.
  *   - The launch's end in few warps.  Once all tickets are drawn, the warps of
  *     a block meet every kTailPasses passes and move their photons together,
  *     so that the long-lived photons do not keep every warp issuing passes for
@@ -36,10 +36,10 @@
  *     memory, so that the loop's state fits the registers.
  *
  * Measured on a GB300 against the transport kernel, calls as a user makes
- * them: 1999 + 2000 strict-math photons 18.9 -> 14.3 ms, 20011 fast photons
- * without the hitting density 4.24 -> 1.93 ms, 1e6 + 2.5e5 photons on 50^3
- * voxels 23.8 -> 11.6 ms, 4e6 wide-field photons on 256 x 256 x 128 voxels
- * 34.3 -> 21.5 ms.  2e7 + 2e7 photons on 128 x 128 x 64 voxels, launches: 105
+ * them: 1999 + 2000 strict-math photons 17.6 -> 13.2 ms, 20011 fast photons
+ * without the hitting density 4.64 -> 2.08 ms, 1e6 + 2.5e5 photons on 50^3
+ * voxels 23.8 -> 11.5 ms, 4e6 wide-field photons on 256 x 256 x 128 voxels
+ * 34.5 -> 21.6 ms.  2e7 + 2e7 photons on 128 x 128 x 64 voxels, launches: 105
  * -> 85 ms and 169 -> 124 ms.  On 200 x 200 x 100 voxels (256 x 5) 175 and 140
  * instead of 213 and 190 warp instructions per 32 passes, 84 and 82 % of the
  * issue slots used.
@@ -74,11 +74,7 @@ __device__ __forceinline__ real walk_no_step() { return (real)__int_as_float(0xf
  * lane's pass may run as the common pass or in the event code, by what the
  * other lanes of its warp do, and both have to give the same bits.  In strict
  * math a multiply-add is two roundings, as on the host. */
-#if MCFL_F64
-__device__ __forceinline__ real fp_mul(real a, real b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ real fp_add(real a, real b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ real fp_fma(real a, real b, real c) { return __fma_rn(a, b, c); }
-#elif MCFL_EXACT_MATH
+#if MCFL_EXACT_MATH
 __device__ __forceinline__ real fp_mul(real a, real b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ real fp_add(real a, real b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ real fp_fma(real a, real b, real c) { return __fadd_rn(__fmul_rn(a, b), c); }
@@ -93,8 +89,9 @@ __device__ __forceinline__ real fp_one_minus_sq(real v) { return fp_fma(-v, v, M
 
 /* spin() with the azimuth's sine and cosine, q = 1 - dz^2 and the uniform
  * given.  kAxis: the direction can lie on the z axis.  kSplit:
- * sin(theta)^2 with two roundings, as the 128 x 9 shape has always had it in
- * fast math (its results and the others' agree statistically). */
+ * sin(theta)^2 with two roundings, as the transport kernel's 128 x 9 shape has
+ * it in fast math: runs in that shape keep their tallies, which differ from the
+ * other shapes' (they agree statistically). */
 template <bool kAxis, bool kSplit>
 __device__ __forceinline__ void walk_spin(Photon &p, const Rec &c, real u_hg, real cosp, real sinp, real q) {
   const real two_g = c.b.x;
@@ -186,8 +183,8 @@ __device__ __forceinline__ bool walk_reflect(Photon &p, real n1, real n2, Rng &r
   return true;
 }
 
-/* The end point of a step, its grid index (clamped: always a voxel) and
- * whether the index is the point's. */
+/* The x-fastest grid index of a point, clamped: always a voxel, the point's own
+ * where the point lies in the grid. */
 __device__ __forceinline__ uint32_t walk_voxel(const Med &m, real x, real y, real z) {
   const uint32_t i = MCFL_R2U_RZ(fp_mul(fp_add(x, m.hx), m.gx)) +
                      m.nx * (MCFL_R2U_RZ(fp_mul(fp_add(y, m.hy), m.gy)) + m.ny * MCFL_R2U_RZ(fp_mul(z, m.gz)));
@@ -547,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) MCFL_WALK_NAME(McflLaunc
                   fnl = walk_depth(fr);
                   /* a beam starts along the z axis, where the deflection has
                    * a form of its own: its first pass, when it is common
-                   * otherwise, is made here, by all lanes */
+                   * otherwise, is made here, for all the photons set up */
                   const real fs = fp_mul(fnl, s_lab[2 * f.label].x), fz = fp_fma(fs, f.dz, f.z);
                   const real fq = fp_one_minus_sq(f.dz);
                   if (!kTime && !(fq > MCFL_C(0.0)) && fminf(fz, fs) > MCFL_C(0.0) && fz < m.esp && f.weight > w_event &&

@@ -323,20 +323,28 @@ const char *mcfl_last_error(void);
 /* Options: "math" (MCFL_MATH_*), "block" (threads per block, at most the
  * variant's bound), "variant" (occupancy variant of the single-medium kernel:
  * 0 = 256 threads x 4 blocks per SM, 1 = 256 x 5, 2 = 128 x 9; setting it
- * also resets "variant_fl"), "variant_fl" (the emission phase's own
- * occupancy variant in mcfl_run; -1: as "variant"),
+ * also resets "variant_fl"; in fast math the 128 x 9 shape rounds one step of
+ * the deflection in another way than the others, so its tallies differ from
+ * theirs, statistically equal, and a run that is to be repeated bit for bit
+ * sets the variants itself instead of taking the autotuner's), "variant_fl" (the
+ * emission phase's own occupancy variant in mcfl_run; -1: as "variant"),
  * "mixed_variant" (occupancy variant of the mixed-media kernel that batches
  * over several media and the server run: 0 = 256 x 3, 1 = 256 x 4, the
  * default, 2 = 128 x 7),
  * "blocks_per_sm" (0 = occupancy maximum), "step_cap" (passes per photon),
- * "l2_window" (1: persisting L2 access window on the labels and tallies),
+ * "l2_window" (1: persisting L2 access window on the label array that a
+ * single-medium launch reads in every pass),
  * "phd_agg" (the photon-hitting-density tally of the single-medium kernel:
- * 0 one atomic add per pass; 1 a thread's successive passes in one voxel
- * summed in a register before the add; 2 the adds of a warp's lanes summed
- * per voxel, one add per distinct voxel; the tallies are the same),
+ * 0 the kernel's own form, one atomic add per pass or, on media with one
+ * refractive index and few voxels under the source, a thread's successive
+ * passes in one voxel summed first; 1 and 2 run the general kernel: 1 a
+ * thread's successive passes in one voxel summed in a register before the
+ * add; 2 the adds of a warp's lanes summed per voxel, one add per distinct
+ * voxel; in strict math the tallies are the same),
  * "pass_form" (0: the single-medium pass arranged for the SIMT warp, the
  * common case straight-line and every rare case behind one branch; 1: every
- * test of the reference's pass as its own branch; the tallies are the same),
+ * test of the reference's pass as its own branch, in the general kernel; in
+ * strict math the tallies are the same),
  * "relaunch" (1..32: the lanes of a warp whose photons ended wait until at
  * least this many of them are free, or the warp's tickets are gone, and
  * then start their next photons together; 1 starts each photon as soon as
@@ -383,7 +391,7 @@ size_t mcfl_medium_bytes(const mcfl_medium *medium);
 int mcfl_medium_from_simulation(mcfl_ctx *ctx, const mcfl_simulation *sim, mcfl_medium **medium);
 
 /* Times every kernel variant with and without the L2 window, with each form
- * of the pass, with "relaunch" 1 and 2 for the SIMT-arranged pass, and (when
+ * of the pass, with "relaunch" 1 and 2 for the default pass, and (when
  * the run tallies the photon hitting density) with each form of that tally,
  * on a sample of `run` (sample_photons excitation photons,
  * photons_per_voxel scaled by the same fraction) and keeps the fastest in
